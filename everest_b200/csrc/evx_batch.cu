@@ -2,8 +2,8 @@
 // persistent launch per motif size (include/everest_b200.h, evx_batch_*).
 //
 // The queries are ordered by motif size (stable); each size's queries form
-// one device work queue: their root ranges are cut into tiles of tile_roots
-// roots laid end to end, warps claim tiles with one atomicAdd and switch
+// one device work queue: their root ranges are cut into tiles of at most
+// tile_roots roots laid end to end, warps claim tiles with one atomicAdd and switch
 // their per-warp query copy when a tile belongs to another query, so cheap
 // and expensive queries share the GPU without per-query tails or per-query
 // launches.  Each size runs the kernel instantiated for exactly that size
@@ -56,8 +56,8 @@ namespace {
 
 constexpr int kCursors = 8;  // one work-queue cursor word per motif size
 // a motif-size group of the table: {k, first table position, queries, tiles,
-// grid, pair-run walk (0/1)}
-constexpr int kGroupWords = 6;
+// grid, pair-run walk (0/1), roots per tile}
+constexpr int kGroupWords = 7;
 
 void drop_exec(evx_batch *b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -80,7 +80,7 @@ int enqueue(evx_batch *b, int nq) {
     la.table = b->table_d + beg;
     la.nq = n;
     la.total_tiles = tiles;
-    la.tile_roots = b->tile_roots;
+    la.tile_roots = b->groups[gi + 6];
     la.cursor = reinterpret_cast<int *>(b->counts_d + b->max_q + gi / kGroupWords);
     la.counts = b->counts_d + beg;
     la.limit = b->limit;
@@ -234,22 +234,28 @@ int evx_batch_launch(evx_batch *b) {
   for (int pos = 0; pos < nq;) {
     const int k = b->queries[b->order[pos]].plan.k;
     const int beg = pos;
-    int tiles = 0;
+    long long roots = 0;
     bool ps = false;
     for (; pos < nq && b->queries[b->order[pos]].plan.k == k; pos++) {
-      QueryDesc q = b->queries[b->order[pos]];
+      const QueryDesc &q = b->queries[b->order[pos]];
       ps = ps || plan_pair_scan(q.plan, q.flags, false);
-      q.tile_beg = tiles;
-      const int n = q.root_end - q.root_beg;
-      tiles += n > 0 ? (n + b->tile_roots - 1) / b->tile_roots : 0;
-      b->table_h[pos] = q;
+      roots += std::max(0, q.root_end - q.root_beg);
     }
     int bps = 0;
     int rc = table_occupancy(k, ps, &bps);  // also sets the kernel attributes before any capture
     if (rc) return rc;
     if (b->blocks_per_sm > 0) bps = b->blocks_per_sm;
     if (bps < 1) bps = 1;
-    b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0});
+    const int tile_roots = tile_roots_for(k, roots, bps * b->num_sms, b->tile_roots);
+    int tiles = 0;
+    for (int i = beg; i < pos; i++) {
+      QueryDesc q = b->queries[b->order[i]];
+      q.tile_beg = tiles;
+      const int n = q.root_end - q.root_beg;
+      tiles += n > 0 ? (n + tile_roots - 1) / tile_roots : 0;
+      b->table_h[i] = q;
+    }
+    b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots});
     launches += tiles > 0 ? 1 : 0;
   }
   if ((int)b->groups.size() / kGroupWords > kCursors)

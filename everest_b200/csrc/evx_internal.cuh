@@ -158,8 +158,8 @@ struct LaunchArgs {
   const QueryDesc *table;     // device table (nq > 1); ignored when nq == 1
   int nq;
   int total_tiles;
-  int tile_roots;             // roots per tile (multiple of 32)
-  int *cursor;                // next unclaimed tile
+  int tile_roots;             // roots per tile
+  int *cursor;                // tiles claimed past each warp's first one
   unsigned long long *counts; // [nq] per-query counts
   unsigned long long limit;   // work limit per query (0 = none): a query whose
                               // meter passes it is stopped early
@@ -247,6 +247,9 @@ int cuda_fail(cudaError_t e, const char *what);
     cudaError_t _e = (call);                             \
     if (_e != cudaSuccess) return ::evx::cuda_fail(_e, #call); \
   } while (0)
+
+// Roots per tile of a k-edge launch of `grid` blocks over `roots` roots, `most` at most.
+int tile_roots_for(int k, long long roots, int grid, int most);
 
 // Launch the search for one query (defined in evx_search.cu).
 int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args,

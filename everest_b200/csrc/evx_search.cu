@@ -42,6 +42,7 @@
 //  * enumeration slots are reserved with one warp-aggregated atomicAdd per
 //    step (the reference issues one atomicAdd per match,
 //    system/tmine/KernelGen.py:505-524).
+#include <algorithm>
 #include <atomic>
 
 #include "evx_internal.cuh"
@@ -298,6 +299,7 @@ struct alignas(16) WarpSmem {
   int4 root[32];
   int4 task[(K > 2) ? (K - 2) : 1][kCap][2];
   int4 save[(K > 2) ? (K - 2) : 1][32][2];
+  int slice[32];           // root batch: lane's share of its root's level-0 range, parts << 16 | part
   int nb[K];
   int cur_q;               // index of the current query in the launch
   int halt;                // set when the current query stops early (limit or cap)
@@ -563,6 +565,7 @@ struct Searcher {
     const int nmc = plan_nm(w);
     int pos = 0, end = 0, want = -1, base = 0;
     int stride = 1;  // distance between this lane's records (interleaved slices)
+    const int share = l == 0 && l < L - 1 ? sm.slice[lane] : 1 << 16;  // of the root (see the kernel)
     bool out = true;
     bool prun = false;  // the range is a run of pair_rec (the edge's static pair), not a list
     int blo = 0, bhi = 0, gstep = 0;
@@ -811,7 +814,8 @@ struct Searcher {
           const bool more = n2 > kRevMax;
           const int4 *lst1 = out ? g.out_rec : g.in_rec;
           if (!more && pos + kRevRatio * n2 < end && ld_t(lst1 + pos + kRevRatio * n2) <= tl) {
-            for (int j = 0; j < n2; j++) {
+            const bool first = l > 0 || (share & 0xffff) == 0;  // a shared root is counted once
+            for (int j = 0; first && j < n2; j++) {
               const int4 c3 = __ldg(lst + lo + j);
               const int cn = c3.y;
               bool fresh = true;
@@ -823,10 +827,14 @@ struct Searcher {
                 cnt += (unsigned long long)pair_count_eids(g, f.x, f.y, p.eid + 1, c3.x - 1);
               }
             }
-            cand += (unsigned)(n2 + 1);
+            if (first) cand += (unsigned)(n2 + 1);
             pos = end;
           }
         }
+      }
+      if (l == 0) {
+        pos += share & 0xffff;
+        stride = share >> 16;
       }
       int chk = 0;
       while (true) {
@@ -1162,14 +1170,19 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
       if (la.limit) S.meter_add();
     }
   };
+  // a warp's first tile is the one of its number, the cursor hands out the
+  // others: the warps of a launch do not meet at the cursor when they start
+  const int warps = (int)(gridDim.x * kWarps);
+  int next = (int)(blockIdx.x * kWarps + (threadIdx.x >> 5));
   while (true) {
-    int t = 0;
+    int t = next;
     if (lane == 0) {
       if (ENUM && *(volatile int *)ea.stop) t = la.total_tiles;
-      else t = atomicAdd(la.cursor, 1);
+      else if (t < 0) t = atomicAdd(la.cursor, 1) + warps;
     }
     t = __shfl_sync(kFull, t, 0);
     if (t >= la.total_tiles) break;
+    next = -1;
     // query of this tile
     int q = 0;
     if (la.table != nullptr && la.nq > 1) {
@@ -1264,6 +1277,22 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
         n += take;
         b0 += adv;
       }
+      // A batch of few roots (the end of a tile, the small tiles of a short
+      // root range) gives each root to 2, 4, .. 32 lanes, which deal its
+      // level-0 range out between them record by record, as in a rebalance
+      // (1000 roots of a 4-cycle: 62 -> 53 us; the 36 three-edge queries on
+      // 7.8M edges: 37.8 -> 37.3 ms).
+      int sh = 0;
+      if (EVX_STRIDED && K > 2 && n > 0 && n <= 16 && S.si) {
+        sh = __clz(n - 1) - 27;  // n << sh is the most lanes that fit
+        if (n == 1) sh = 5;
+        __syncwarp();
+        const int4 rt = sm.root[lane >> sh];
+        __syncwarp();
+        sm.root[lane] = rt;
+        n <<= sh;
+      }
+      if (K > 2) sm.slice[lane] = (1 << (16 + sh)) | (lane & ((1 << sh) - 1));
       const bool has = lane < n;
       __syncwarp();
       if (!ENUM && S.kr() == 2 && (S.qf & kQInlineLast)) {
@@ -1349,8 +1378,6 @@ QueryDesc single_query(const MotifPlan &plan, const SearchArgs &args) {
   return q;
 }
 
-constexpr int kSingleTileRoots = 64;
-
 }  // namespace
 
 // single-query launches: exact motif size, count or enumerate, with or
@@ -1388,6 +1415,25 @@ bool plan_pair_scan(const MotifPlan &plan, int qflags, bool enumerate) {
   return false;
 }
 
+// A tile is what one warp searches alone, so it decides how evenly a launch
+// ends: 64 roots (32 leave batches short after the window bound: the 36
+// three-edge queries on 7.8M edges 37.3 -> 39.8 ms; six five-edge queries on
+// 1.3M edges 2.07 -> 2.09 ms), but 32 for four edges (the 4-cycle on 36M edges
+// 132.9 -> 127.3 ms; 16: 133.2 ms).  A root range too short to give every
+// warp several of those is cut finer.  Up to three edges, down to one tile per
+// warp and no further: a batch costs its latency however few its roots
+// (triangle on 200k edges: 198 us with tiles of 64, 119 with one tile per warp,
+// 163 with four).  More edges, eight tiles per warp of 16 roots or more, since
+// a root's cost varies more (500k roots of the 4-cycle: 2.50 ms with tiles of
+// 64, 1.70 ms with 16, 1.65 ms with 8; four light edges on 321k edges: 149 us
+// with 64, 131 with 19, 179 with 9).
+int tile_roots_for(int k, long long roots, int grid, int most) {
+  const long long per_warp = roots / ((long long)grid * kWarps);
+  const long long t = k <= 3 ? per_warp : std::max(per_warp / 8, std::min(per_warp, 16ll));
+  const long long least = k == 2 ? 32 : 1;  // (two edges: a batch's lanes are not shared, 60 against 64 us on 199k edges)
+  return (int)std::max(least, std::min(t, (long long)std::min(most, k == 4 ? 32 : 64)));
+}
+
 int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args, int grid, int block,
                   cudaStream_t stream) {
   (void)block;
@@ -1397,9 +1443,9 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
   LaunchArgs la{};
   la.table = nullptr;
   la.nq = 1;
-  la.tile_roots = kSingleTileRoots;
   const int n = args.root_end - args.root_beg;
-  la.total_tiles = n > 0 ? (n + kSingleTileRoots - 1) / kSingleTileRoots : 0;
+  la.tile_roots = tile_roots_for(k, n, grid, n);
+  la.total_tiles = n > 0 ? (n + la.tile_roots - 1) / la.tile_roots : 0;
   la.cursor = args.cursor;
   la.counts = args.count;
   la.limit = args.limit;
