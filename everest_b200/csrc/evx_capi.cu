@@ -26,7 +26,7 @@ int cuda_fail(cudaError_t e, const char *what) {
   return fail(e == cudaErrorMemoryAllocation ? EVX_ERR_NOMEM : EVX_ERR_CUDA, m);
 }
 
-int graph_t_range(DeviceGraph &g, int *scratch_d, cudaStream_t s);
+int graph_t_range(DeviceGraph &g, int *scratch_d, bool *in_grouped, cudaStream_t s);
 
 namespace {
 std::mutex g_pool_mu;
@@ -237,10 +237,12 @@ static int alloc_graph(int device, int64_t E, int64_t V, evx_graph **out, cudaSt
   A((void **)&g.out_rec, sizeof(int4) * e1);
   A((void **)&g.in_rec, sizeof(int4) * e1);
   A((void **)&g.node_rng, sizeof(int4) * (size_t)(V > 0 ? V : 1));
+  A((void **)&g.sig_out, sizeof(unsigned long long) * (size_t)(V > 0 ? V : 1));
+  A((void **)&g.sig_in, sizeof(unsigned long long) * (size_t)(V > 0 ? V : 1));
   g.bytes = (int64_t)bytes;
   if (err != cudaSuccess) {
     dev_free(g.edges, s); dev_free(g.inpos, s); dev_free(g.euid, s); dev_free(g.out_rec, s);
-    dev_free(g.in_rec, s); dev_free(g.node_rng, s);
+    dev_free(g.in_rec, s); dev_free(g.node_rng, s); dev_free(g.sig_out, s); dev_free(g.sig_in, s);
     delete h;
     return cuda_fail(err, "device graph allocation");
   }
@@ -249,12 +251,26 @@ static int alloc_graph(int device, int64_t E, int64_t V, evx_graph **out, cudaSt
   return EVX_OK;
 }
 
-static int finish_graph(evx_graph *h, cudaStream_t s) {
-  int *scratch = nullptr;
-  EVX_CUDA(dev_alloc((void **)&scratch, 2 * sizeof(int), h->g.device, s));
-  int rc = graph_t_range(h->g, scratch, s);
-  dev_free(scratch, s);
-  if (!rc) rc = build_pair_index(h->g, s);
+// Checks and packs the host-format arrays on the device; *scratch (for
+// finish_graph) holds the time range, the in-list flag and the list nodes.
+static ListScratch list_scratch(const DeviceGraph &g, int *scratch) {
+  return ListScratch{scratch + 32, scratch + 32 + g.num_edges, scratch + 2};
+}
+
+static int start_graph(evx_graph *h, const int *eg_d, const int *out_v_d, const int *in_v_d, const int *out_r_d,
+                       const int *in_r_d, const int *euid_d, int **scratch, cudaStream_t s) {
+  DeviceGraph &g = h->g;
+  int rc = validate_graph(g.device, g.num_edges, g.num_vertices, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, s);
+  if (rc) return rc;
+  EVX_CUDA(dev_alloc((void **)scratch, (32 + 2 * (size_t)g.num_edges) * sizeof(int), g.device, s));
+  EVX_CUDA(cudaMemsetAsync(*scratch, 0, 32 * sizeof(int), s));
+  return pack_graph(g, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, euid_d, list_scratch(g, *scratch), s);
+}
+
+static int finish_graph(evx_graph *h, int *scratch, cudaStream_t s) {
+  bool in_grouped = false;
+  int rc = graph_t_range(h->g, scratch, &in_grouped, s);
+  if (!rc) rc = build_pair_index(h->g, list_scratch(h->g, scratch), in_grouped, s);
   if (!rc) {
     EVX_CUDA(cudaStreamSynchronize(s));
   }
@@ -269,9 +285,10 @@ int evx_graph_from_device(int device, int64_t num_edges, int64_t num_vertices, c
     return fail(EVX_ERR_INVALID, "null graph array");
   int rc = alloc_graph(device, num_edges, num_vertices, out, s);
   if (rc) return rc;
-  rc = validate_graph(device, num_edges, num_vertices, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, s);
-  if (!rc) rc = pack_graph((*out)->g, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, euid_d, s);
-  if (!rc) rc = finish_graph(*out, s);
+  int *scratch = nullptr;
+  rc = start_graph(*out, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, euid_d, &scratch, s);
+  if (!rc) rc = finish_graph(*out, scratch, s);
+  dev_free(scratch, s);
   if (rc) { evx_graph_free(*out); *out = nullptr; }
   return rc;
 }
@@ -312,10 +329,11 @@ int evx_graph_upload(int device, int64_t num_edges, int64_t num_vertices, const 
   C(ir_d, in_r, sizeof(int) * V1);
   if (euid) C(eu_d, euid, sizeof(int) * ne);
   // the packing kernels index with these arrays: check them on the device first
-  if (!rc) rc = validate_graph(device, num_edges, num_vertices, eg_d, ov_d, iv_d, or_d, ir_d, s);
-  if (!rc) rc = pack_graph((*out)->g, eg_d, ov_d, iv_d, or_d, ir_d, euid ? eu_d : nullptr, s);
+  int *scratch = nullptr;
+  if (!rc) rc = start_graph(*out, eg_d, ov_d, iv_d, or_d, ir_d, euid ? eu_d : nullptr, &scratch, s);
   dev_free(buf, s);
-  if (!rc) rc = finish_graph(*out, s);
+  if (!rc) rc = finish_graph(*out, scratch, s);
+  dev_free(scratch, s);
   cudaStreamSynchronize(s);
   if (rc) { evx_graph_free(*out); *out = nullptr; }
   return rc;

@@ -299,8 +299,16 @@ int cons_check_program(const evx_program &p, int num_vars, const char *what);
 int cons_build_masks(const evx_constraints &c, int n, const int *node_feat, int V, const int *edge_feat,
                      int E, unsigned short *node_ok, unsigned char *edge_ok, int num_sms, cudaStream_t s);
 
-// Build the pair index (defined in evx_pairs.cu); needs edges[] packed.
-int build_pair_index(DeviceGraph &g, cudaStream_t s);
+// What packing leaves for the pair index build: the node of each position of
+// the out- and in-lists, and whether an in-list entry is out of place.
+struct ListScratch {
+  int *out_node, *in_node;  // [E]
+  int *stray;
+};
+
+// Build the pair index (defined in evx_pairs.cu); needs the packed graph.
+// in_grouped: in_rec is in (target, edge id) order.
+int build_pair_index(DeviceGraph &g, const ListScratch &lists, bool in_grouped, cudaStream_t s);
 
 // Check the host-format arrays on the device before anything indexes with
 // them (evx_graph.cu); returns EVX_ERR_INVALID with a message on bad input.
@@ -308,9 +316,9 @@ int validate_graph(int device, int64_t E, int64_t V, const int *eg_d, const int 
                    const int *out_r_d, const int *in_r_d, cudaStream_t s);
 
 // Build the packed device layout from the uploaded host-format arrays
-// (defined in evx_graph.cu).
+// (defined in evx_graph.cu) and fill lists (*lists.stray: zero before).
 int pack_graph(DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *in_v_d,
-               const int *out_r_d, const int *in_r_d, const int *euid_d, cudaStream_t s);
+               const int *out_r_d, const int *in_r_d, const int *euid_d, const ListScratch &lists, cudaStream_t s);
 
 }  // namespace evx
 
