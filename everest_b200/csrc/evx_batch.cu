@@ -1,7 +1,7 @@
 // Batched queries: many count queries against one resident graph in one
 // persistent launch per motif size (include/everest_b200.h, evx_batch_*).
 //
-// The queries are ordered by motif size (stable); each size's queries form
+// The queries are ordered by motif size; each size's queries form
 // one device work queue: their root ranges are cut into tiles of at most
 // tile_roots roots laid end to end, warps claim tiles with one atomicAdd and switch
 // their per-warp query copy when a tile belongs to another query, so cheap
@@ -10,6 +10,13 @@
 // (its levels are compile-time).  The launch sequence (query table upload,
 // counter reset, the kernels, counts read-back) is captured once into a CUDA
 // graph and replayed while the batch keeps the same shape.
+//
+// The sizes' kernels run side by side, the largest motifs first, and a size's
+// queries start with the widest time windows: a launch ends with a few warps
+// on its heaviest roots, whose SMs the next size's blocks then fill, and the
+// heaviest roots start early (64 mixed queries over windows of 250k roots,
+// one size after the other and in the given order: 30.0 ms; side by side, widest
+// first: 23.4 ms; 64 requests over windows of 1000 roots: 0.61 -> 0.45 ms).
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -20,6 +27,10 @@
 #include "evx_internal.cuh"
 
 using namespace evx;
+
+namespace {
+constexpr int kSizes = EVX_MAX_MOTIF_EDGES - 1;  // motif sizes, each a launch of its own
+}
 
 struct evx_batch {
   int device = 0;
@@ -34,6 +45,8 @@ struct evx_batch {
   unsigned long long *counts_d = nullptr;  // [max_q] counts, kCursors cursor words, [max_q] work meters
   unsigned long long *counts_h = nullptr;  // pinned [max_q] counts, [max_q] meters
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaStream_t side[kSizes - 1] = {};      // streams of the second and later sizes
+  cudaEvent_t fork = nullptr, join[kSizes - 1] = {};
   // tuning
   int tile_roots = 256, blocks_per_sm = 0, steal_interval = 16, min_split = 2, use_graph = 1;
   unsigned long long limit = 0;  // work limit per query (0 = none)
@@ -55,6 +68,7 @@ struct evx_batch {
 namespace {
 
 constexpr int kCursors = 8;  // one work-queue cursor word per motif size
+static_assert(kSizes <= kCursors, "a cursor per motif size");
 // a motif-size group of the table: {k, first table position, queries, tiles,
 // grid, pair-run walk (0/1), roots per tile}
 constexpr int kGroupWords = 7;
@@ -71,24 +85,36 @@ int enqueue(evx_batch *b, int nq) {
                            b->stream));
   EVX_CUDA(cudaMemsetAsync(b->counts_d, 0, sizeof(unsigned long long) * (2 * (size_t)b->max_q + kCursors),
                            b->stream));
-  for (size_t gi = 0; gi < b->groups.size(); gi += kGroupWords) {
-    const int k = b->groups[gi], beg = b->groups[gi + 1], n = b->groups[gi + 2];
-    const int tiles = b->groups[gi + 3], grid = b->groups[gi + 4];
-    const bool ps = b->groups[gi + 5] != 0;
-    if (tiles <= 0) continue;
-    LaunchArgs la{};
-    la.table = b->table_d + beg;
-    la.nq = n;
-    la.total_tiles = tiles;
-    la.tile_roots = b->groups[gi + 6];
-    la.cursor = reinterpret_cast<int *>(b->counts_d + b->max_q + gi / kGroupWords);
-    la.counts = b->counts_d + beg;
-    la.limit = b->limit;
-    la.meter = meter + beg;
-    int rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, ps, grid, b->stream);
-    if (rc) return rc;
-    EVX_CUDA(cudaGetLastError());
+  // the first launch runs on the batch's stream, the others beside it
+  const size_t groups = b->groups.size() / kGroupWords;
+  if (groups > 1) EVX_CUDA(cudaEventRecord(b->fork, b->stream));
+  int rc = EVX_OK;
+  for (size_t gi = 0; gi < groups; gi++) {
+    const int *gr = &b->groups[gi * kGroupWords];
+    const int k = gr[0], beg = gr[1], tiles = gr[3], grid = gr[4];
+    cudaStream_t s = gi ? b->side[gi - 1] : b->stream;
+    if (gi) EVX_CUDA(cudaStreamWaitEvent(s, b->fork, 0));
+    if (tiles > 0 && !rc) {
+      LaunchArgs la{};
+      la.table = b->table_d + beg;
+      la.nq = gr[2];
+      la.total_tiles = tiles;
+      la.tile_roots = gr[6];
+      la.cursor = reinterpret_cast<int *>(b->counts_d + b->max_q + gi);
+      la.counts = b->counts_d + beg;
+      la.limit = b->limit;
+      la.meter = meter + beg;
+      rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, gr[5] != 0, grid, s);
+      cudaError_t e = cudaGetLastError();
+      if (!rc && e != cudaSuccess) rc = cuda_fail(e, "batch search launch");
+    }
+    // joined on errors too: a side stream is never left behind in a capture
+    if (gi) {
+      EVX_CUDA(cudaEventRecord(b->join[gi - 1], s));
+      EVX_CUDA(cudaStreamWaitEvent(b->stream, b->join[gi - 1], 0));
+    }
   }
+  if (rc) return rc;
   EVX_CUDA(cudaMemcpyAsync(b->counts_h, b->counts_d, sizeof(unsigned long long) * (size_t)nq,
                            cudaMemcpyDeviceToHost, b->stream));
   if (b->limit)
@@ -127,6 +153,11 @@ int evx_batch_create(int device, int max_queries, void *stream, evx_batch **out)
   if (e == cudaSuccess) e = cudaMallocHost(&b->counts_h, sizeof(unsigned long long) * 2 * (size_t)max_queries);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
+  for (int i = 0; i < kSizes - 1; i++) {
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
+  }
   if (e != cudaSuccess) {
     evx_batch_destroy(b);
     return cuda_fail(e, "batch setup");
@@ -147,6 +178,11 @@ int evx_batch_destroy(evx_batch *b) {
   if (b->counts_h) cudaFreeHost(b->counts_h);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
+  if (b->fork) cudaEventDestroy(b->fork);
+  for (int i = 0; i < kSizes - 1; i++) {
+    if (b->join[i]) cudaEventDestroy(b->join[i]);
+    if (b->side[i]) cudaStreamDestroy(b->side[i]);
+  }
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return EVX_OK;
@@ -224,11 +260,14 @@ int evx_batch_launch(evx_batch *b) {
   const int nq = (int)b->queries.size();
   if (nq == 0) return fail(EVX_ERR_STATE, "empty batch");
   EVX_CUDA(cudaSetDevice(b->device));
-  // table order: by motif size, stable; one group (and one launch) per size
+  // table order: the largest motifs first, and of one size the widest windows;
+  // one group (and one launch) per size
   b->order.resize(nq);
   for (int i = 0; i < nq; i++) b->order[i] = i;
-  std::stable_sort(b->order.begin(), b->order.end(),
-                   [b](int x, int y) { return b->queries[x].plan.k < b->queries[y].plan.k; });
+  std::stable_sort(b->order.begin(), b->order.end(), [b](int x, int y) {
+    const QueryDesc &p = b->queries[x], &q = b->queries[y];
+    return p.plan.k != q.plan.k ? p.plan.k > q.plan.k : p.delta > q.delta;
+  });
   b->groups.clear();
   int launches = 0;
   for (int pos = 0; pos < nq;) {
@@ -258,7 +297,7 @@ int evx_batch_launch(evx_batch *b) {
     b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots});
     launches += tiles > 0 ? 1 : 0;
   }
-  if ((int)b->groups.size() / kGroupWords > kCursors)
+  if ((int)b->groups.size() / kGroupWords > kSizes)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {

@@ -1424,12 +1424,12 @@ bool plan_pair_scan(const MotifPlan &plan, int qflags, bool enumerate) {
 // warp and no further: a batch costs its latency however few its roots
 // (triangle on 200k edges: 198 us with tiles of 64, 119 with one tile per warp,
 // 163 with four).  More edges, eight tiles per warp of 16 roots or more, since
-// a root's cost varies more (500k roots of the 4-cycle: 2.50 ms with tiles of
+// a root's cost varies more (four for five edges and more; 500k roots of the 4-cycle: 2.50 ms with tiles of
 // 64, 1.70 ms with 16, 1.65 ms with 8; four light edges on 321k edges: 149 us
 // with 64, 131 with 19, 179 with 9).
 int tile_roots_for(int k, long long roots, int grid, int most) {
   const long long per_warp = roots / ((long long)grid * kWarps);
-  const long long t = k <= 3 ? per_warp : std::max(per_warp / 8, std::min(per_warp, 16ll));
+  const long long t = k <= 3 ? per_warp : std::max(per_warp / (k == 4 ? 8 : 4), std::min(per_warp, 16ll));
   const long long least = k == 2 ? 32 : 1;  // (two edges: a batch's lanes are not shared, 60 against 64 us on 199k edges)
   return (int)std::max(least, std::min(t, (long long)std::min(most, k == 4 ? 32 : 64)));
 }
