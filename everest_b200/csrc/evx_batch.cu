@@ -1,22 +1,23 @@
 // Batched queries: many count queries against one resident graph in one
-// persistent launch per motif size (include/everest_b200.h, evx_batch_*).
+// persistent launch per kind of motif (include/everest_b200.h, evx_batch_*).
 //
-// The queries are ordered by motif size; each size's queries form
-// one device work queue: their root ranges are cut into tiles of at most
-// tile_roots roots laid end to end, warps claim tiles with one atomicAdd and switch
-// their per-warp query copy when a tile belongs to another query, so cheap
-// and expensive queries share the GPU without per-query tails or per-query
-// launches.  Each size runs the kernel instantiated for exactly that size
-// (its levels are compile-time).  The launch sequence (query table upload,
-// counter reset, the kernels, counts read-back) is captured once into a CUDA
-// graph and replayed while the batch keeps the same shape.
+// The queries are ordered by motif size and by how their last edge is counted;
+// each such group forms one device work queue: the root ranges are cut into
+// tiles of at most tile_roots roots laid end to end, warps claim tiles with one
+// atomicAdd and switch their per-warp query copy when a tile belongs to another
+// query, so cheap and expensive queries share the GPU without per-query tails
+// or per-query launches.  Each group runs the kernel compiled for exactly that
+// size and way (64 mixed queries over 250k-root windows: 20.8 ms, against 23.1
+// with one kernel per size).  The launch sequence (query table upload, counter
+// reset, the kernels, counts read-back) is captured once into a CUDA graph and
+// replayed while the batch keeps the same shape.
 //
-// The sizes' kernels run side by side, the largest motifs first, and a size's
-// queries start with the widest time windows: a launch ends with a few warps
-// on its heaviest roots, whose SMs the next size's blocks then fill, and the
-// heaviest roots start early (64 mixed queries over windows of 250k roots,
-// one size after the other and in the given order: 30.0 ms; side by side, widest
-// first: 23.4 ms; 64 requests over windows of 1000 roots: 0.61 -> 0.45 ms).
+// The groups' kernels run side by side, the largest motifs first, and a group's
+// queries start with the widest time windows: a launch ends with a few warps on
+// its heaviest roots, whose SMs the next group's blocks then fill, and the
+// heaviest roots start early (the same 64 queries, one size after the other and
+// in the given order: 30.0 ms; side by side, widest first: 23.4 ms; 64 requests
+// over windows of 1000 roots: 0.61 -> 0.45 ms).
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -67,11 +68,12 @@ struct evx_batch {
 
 namespace {
 
-constexpr int kCursors = 8;  // one work-queue cursor word per motif size
-static_assert(kSizes <= kCursors, "a cursor per motif size");
-// a motif-size group of the table: {k, first table position, queries, tiles,
-// grid, pair-run walk (0/1), roots per tile}
-constexpr int kGroupWords = 7;
+// one work-queue cursor word per launch: motif sizes x ways of counting the
+// last edge (five, and the kernel that holds all)
+constexpr int kCursors = kSizes * 6;
+// a launch's group of the table: {k, first table position, queries, tiles,
+// grid, pair-run walk (0/1), roots per tile, way of counting the last edge}
+constexpr int kGroupWords = 8;
 
 void drop_exec(evx_batch *b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -92,7 +94,8 @@ int enqueue(evx_batch *b, int nq) {
   for (size_t gi = 0; gi < groups; gi++) {
     const int *gr = &b->groups[gi * kGroupWords];
     const int k = gr[0], beg = gr[1], tiles = gr[3], grid = gr[4];
-    cudaStream_t s = gi ? b->side[gi - 1] : b->stream;
+    const size_t si = gi ? (gi - 1) % (kSizes - 1) : 0;
+    cudaStream_t s = gi ? b->side[si] : b->stream;
     if (gi) EVX_CUDA(cudaStreamWaitEvent(s, b->fork, 0));
     if (tiles > 0 && !rc) {
       LaunchArgs la{};
@@ -104,15 +107,15 @@ int enqueue(evx_batch *b, int nq) {
       la.counts = b->counts_d + beg;
       la.limit = b->limit;
       la.meter = meter + beg;
-      rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, gr[5] != 0, grid, s);
+      rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, gr[7], gr[5] != 0, grid, s);
       cudaError_t e = cudaGetLastError();
       if (!rc && e != cudaSuccess) rc = cuda_fail(e, "batch search launch");
     }
-    // joined on errors too: a side stream is never left behind in a capture
-    if (gi) {
-      EVX_CUDA(cudaEventRecord(b->join[gi - 1], s));
-      EVX_CUDA(cudaStreamWaitEvent(b->stream, b->join[gi - 1], 0));
-    }
+  }
+  // joined on errors too: a side stream is never left behind in a capture
+  for (size_t i = 0; i + 1 < groups && i < kSizes - 1; i++) {
+    EVX_CUDA(cudaEventRecord(b->join[i], b->side[i]));
+    EVX_CUDA(cudaStreamWaitEvent(b->stream, b->join[i], 0));
   }
   if (rc) return rc;
   EVX_CUDA(cudaMemcpyAsync(b->counts_h, b->counts_d, sizeof(unsigned long long) * (size_t)nq,
@@ -260,28 +263,32 @@ int evx_batch_launch(evx_batch *b) {
   const int nq = (int)b->queries.size();
   if (nq == 0) return fail(EVX_ERR_STATE, "empty batch");
   EVX_CUDA(cudaSetDevice(b->device));
-  // table order: the largest motifs first, and of one size the widest windows;
-  // one group (and one launch) per size
+  // table order: the largest motifs first, and of one launch the widest
+  // windows; one group (and one launch) per size and way of counting the last
+  // edge
+  const auto tail = [](const QueryDesc &q) { return tail_of(q.plan.k, q.flags); };
   b->order.resize(nq);
   for (int i = 0; i < nq; i++) b->order[i] = i;
-  std::stable_sort(b->order.begin(), b->order.end(), [b](int x, int y) {
+  std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {
     const QueryDesc &p = b->queries[x], &q = b->queries[y];
-    return p.plan.k != q.plan.k ? p.plan.k > q.plan.k : p.delta > q.delta;
+    if (p.plan.k != q.plan.k) return p.plan.k > q.plan.k;
+    const int tp = tail(p), tq = tail(q);
+    return tp != tq ? tp < tq : p.delta > q.delta;
   });
   b->groups.clear();
   int launches = 0;
   for (int pos = 0; pos < nq;) {
-    const int k = b->queries[b->order[pos]].plan.k;
+    const int k = b->queries[b->order[pos]].plan.k, way = tail(b->queries[b->order[pos]]);
     const int beg = pos;
     long long roots = 0;
     bool ps = false;
-    for (; pos < nq && b->queries[b->order[pos]].plan.k == k; pos++) {
+    for (; pos < nq && b->queries[b->order[pos]].plan.k == k && tail(b->queries[b->order[pos]]) == way; pos++) {
       const QueryDesc &q = b->queries[b->order[pos]];
       ps = ps || plan_pair_scan(q.plan, q.flags, false);
       roots += std::max(0, q.root_end - q.root_beg);
     }
     int bps = 0;
-    int rc = table_occupancy(k, ps, &bps);  // also sets the kernel attributes before any capture
+    int rc = table_occupancy(k, way, ps, &bps);  // also sets the kernel attributes before any capture
     if (rc) return rc;
     if (b->blocks_per_sm > 0) bps = b->blocks_per_sm;
     if (bps < 1) bps = 1;
@@ -294,10 +301,10 @@ int evx_batch_launch(evx_batch *b) {
       tiles += n > 0 ? (n + tile_roots - 1) / tile_roots : 0;
       b->table_h[i] = q;
     }
-    b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots});
+    b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots, way});
     launches += tiles > 0 ? 1 : 0;
   }
-  if ((int)b->groups.size() / kGroupWords > kSizes)
+  if ((int)b->groups.size() / kGroupWords > kCursors)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {

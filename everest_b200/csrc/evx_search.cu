@@ -106,15 +106,30 @@ constexpr int kScanWide = EVX_SCAN_WIDE;
 #define EVX_ROOT_PACK 1
 #endif
 
-// resident blocks per SM the register budget aims for (deeper motifs keep
-// more per-level state live)
+// How a kernel counts the last edge: its kQ* bit where that is compiled in
+// (count mode, no strict timestamps, no constraints), kTailAny where the
+// query's flags say (everything else).  A kernel that holds every way spills
+// (196 bytes of stores for 3 edges, 0 to 88 with one way), and its dead paths
+// cost issue slots: the 36 three-edge queries on 7.8M edges 37.2 -> 30.2 ms.
+constexpr int kTailFlags = kQStrict | kQInlineLast | kQSamePair | kQRevPair | kQPairHash | kQPairDir | kQNewArith;
+constexpr int kTailAny = -1;
+
+// Resident blocks per SM the register budget aims for (deeper motifs keep more
+// per-level state live).  3 edges: 10 (the 36 queries 30.2 ms; 8: 32.9, 11 and
+// 12: 31.2).  4 edges: with one way of counting the last edge 8 (the 4-cycle
+// on 36M edges 113.7 ms; 7: 118.5, 9: 118.4), with every way 7.  5 edges: 5
+// with one way (eight new-node queries 1.78 ms; 4: 1.95, 6: 1.95).
 #ifndef EVX_MINB3
 #define EVX_MINB3 10
 #endif
 #ifndef EVX_MINB4
 #define EVX_MINB4 7
 #endif
-constexpr int min_blocks(int k) { return k <= 3 ? EVX_MINB3 : (k == 4 ? EVX_MINB4 : 4); }
+constexpr int min_blocks(int k, int tail) {
+  if (k <= 3) return EVX_MINB3;
+  if (k == 4) return tail < 0 ? EVX_MINB4 : 8;
+  return k == 5 && tail >= 0 ? 5 : 4;
+}
 
 template <int N>
 __device__ __forceinline__ int sel(const int (&a)[N], int i) {
@@ -310,7 +325,7 @@ struct Prev {
   int eid, t, src, dst, pop, pip;
 };
 
-template <int K, bool ENUM, bool EXACT, bool PS, bool CS>
+template <int K, bool ENUM, int TAIL, bool PS, bool CS>
 struct Searcher {
   static constexpr int L = K - 1;          // levels; level l opens motif edge l + 1
   static constexpr int N = K + 1;          // motif nodes <= k + 1
@@ -329,10 +344,10 @@ struct Searcher {
   // registers, the rest read from its shared-memory copy
   int qf = 0;
   int si = 0;
-  // motif edges of the current query: K itself when the launch has one
-  // motif size (EXACT), else the table entry's
-  __device__ __forceinline__ int kr() const { return EXACT ? K : sm.q.plan.k; }
-  __device__ __forceinline__ bool strict_() const { return (qf & kQStrict) != 0; }
+  static constexpr int kr() { return K; }  // motif edges
+  // kQ* flags: with TAIL >= 0 the bits of kTailFlags are known at compile time
+  __device__ __forceinline__ int fl() const { return TAIL < 0 ? qf : ((qf & ~kTailFlags) | TAIL); }
+  __device__ __forceinline__ bool strict_() const { return (fl() & kQStrict) != 0; }
   unsigned long long cnt;
   unsigned cand;  // adjacency records examined inside the window since the last meter update
 
@@ -529,7 +544,7 @@ struct Searcher {
     }
 
     // ---------------------------- last level through the pair hash table ----
-    if (!ENUM && (qf & kQPairHash) && l == kr() - 2) {
+    if (!ENUM && (fl() & kQPairHash) && l == kr() - 2) {
       // the closing last edge of each lane's task: one hash probe sequence
       // for its pair's run, then the run's entries after the previous edge
       // and inside the window (runs are short; 32 lanes probe in parallel)
@@ -546,7 +561,7 @@ struct Searcher {
     }
 
     // --------------------------- last level through the pair directory ----
-    if (!ENUM && (qf & kQPairDir) && l == kr() - 2) {
+    if (!ENUM && (fl() & kQPairDir) && l == kr() - 2) {
       // the closing last edge of each lane's task: count its static pair's
       // run inside the window (converged across the batch's 32 tasks)
       if (has) {
@@ -570,7 +585,7 @@ struct Searcher {
     bool prun = false;  // the range is a run of pair_rec (the edge's static pair), not a list
     int blo = 0, bhi = 0, gstep = 0;
     bool searching = false;
-    if (PS && has && kind == 2 && (qf & kQPairScan)) {
+    if (PS && has && kind == 2 && (fl() & kQPairScan)) {
       // both endpoints are mapped: walk the run of the static edge (ia, ib)
       // after the previous edge; every entry matches structurally.  The run
       // is located from the previous edge itself when it is that pair or its
@@ -695,7 +710,7 @@ struct Searcher {
             }
           }
           if constexpr (!ENUM) {
-            if (want < 0 && pos < end && arith && (qf & kQNewArith) && st == 1) {
+            if (want < 0 && pos < end && arith && (fl() & kQNewArith) && st == 1) {
               // a last edge that maps a new node, and the window goes on past
               // this step: when the rest of the window is long, it counts
               // every record except those whose other endpoint is already
@@ -741,11 +756,11 @@ struct Searcher {
       // --------------------------------- scan, queue children, descend ----
       // The level before the last one counts a closing last edge inline by
       // range arithmetic on the pair index (count mode only).
-      const bool inline_here = (l == kr() - 3) && !ENUM && (qf & (kQInlineLast | kQSamePair | kQRevPair));
+      const bool inline_here = (l == kr() - 3) && !ENUM && (fl() & (kQInlineLast | kQSamePair | kQRevPair));
       const int wl = plan.info[kr() - 2];
       const int la = plan_a(wl), lb = plan_b(wl);
       int ca = -1, cb = -1, ctl = 0, cs = 0, cub = 0, ckey = 0;  // this lane's pair cursor
-      if (inline_here && (qf & kQInlineLast) && has && pos < end) {
+      if (inline_here && (fl() & kQInlineLast) && has && pos < end) {
         // the closing pair is fixed for the task: place the cursor on its
         // run's entries after the previous edge inside the window once; when
         // there are none, no candidate of the task can close and its scan is
@@ -774,7 +789,7 @@ struct Searcher {
         if (cs >= cub) pos = end;
       }
       if (l == kr() - 3 && plan_kind(wl) == 2 && (la < nmc) != (lb < nmc) &&
-          !(qf & (kQInlineLast | kQNoPrune)) && has && pos < end && !prun) {
+          !(fl() & (kQInlineLast | kQNoPrune)) && has && pos < end && !prun) {
         // the closing edge has one endpoint mapped before this level, fixed
         // for the task: when that node's list (out-list of a source, in-list
         // of a destination) has no entry after the previous edge inside the
@@ -799,7 +814,7 @@ struct Searcher {
         }
         if (lo >= hi || ld_t(lst + lo) > tl) {
           pos = end;
-        } else if (EVX_REVERSE_CLOSE && !ENUM && !CS && !strict_() && !(qf & (kQSamePair | kQRevPair))) {
+        } else if (EVX_REVERSE_CLOSE && !ENUM && !CS && !strict_() && !(fl() & (kQSamePair | kQRevPair))) {
           // Few closing edges: count the task from the closing side.  Each
           // closing edge e2 (x, c) inside the window pairs with the
           // candidates e1 of this level that map the same new node c and
@@ -926,11 +941,11 @@ struct Searcher {
               }
             }
           }
-          if (qf & (kQSamePair | kQRevPair)) {
+          if (fl() & (kQSamePair | kQRevPair)) {
             // the last edge repeats the matched edge's endpoints (or reverses
             // them): count the entries of that edge's own pair run (or of the
             // reverse pair's run) after the edge and inside the window
-            const bool rev = (qf & kQRevPair) != 0;
+            const bool rev = (fl() & kQRevPair) != 0;
             // a candidate whose record says its own pair's run (top bit) or
             // its reverse pair's run (kRevLater) has no entry after it adds
             // nothing: skip its lookup
@@ -1012,14 +1027,14 @@ struct Searcher {
           }
         }
       }
-      if (EVX_TAIL_QUEUE && inline_here && (qf & (kQSamePair | kQRevPair)) && !strict_()) {
+      if (EVX_TAIL_QUEUE && inline_here && (fl() & (kQSamePair | kQRevPair)) && !strict_()) {
         // the queued tail lookups left over (none when the query stopped)
         if (sm.halt) {
           __syncwarp();
           if (lane == 0) sm.nb[l + 1] = 0;
           __syncwarp();
         } else {
-          tail_batch<l>((qf & kQRevPair) != 0, true);
+          tail_batch<l>((fl() & kQRevPair) != 0, true);
         }
       }
     }
@@ -1145,8 +1160,8 @@ struct Searcher {
 // Persistent search: warps claim root tiles from one work queue covering
 // every query of the launch, switch their per-warp query copy when a tile
 // belongs to another query, and add each query's count to counts[q].
-template <int K, bool ENUM, bool EXACT, bool PS, bool CS>
-__global__ void __launch_bounds__(kBlock, min_blocks(K))
+template <int K, bool ENUM, int TAIL, bool PS, bool CS>
+__global__ void __launch_bounds__(kBlock, min_blocks(K, TAIL))
 search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const LaunchArgs la,
               const __grid_constant__ EnumArgs ea) {
   extern __shared__ int4 dyn_smem[];
@@ -1156,7 +1171,7 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
   if (lane < K) sm.nb[lane] = 0;
   if (lane == 0) { sm.halt = 0; sm.cur_q = 0; }
   __syncwarp();
-  Searcher<K, ENUM, EXACT, PS, CS> S(g, sm.q.plan, ea, la, sm, lane);
+  Searcher<K, ENUM, TAIL, PS, CS> S(g, sm.q.plan, ea, la, sm, lane);
   int cur_q = -1;
   auto flush = [&]() {
     if (cur_q >= 0) {
@@ -1223,7 +1238,7 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
     // at a root node): 0 / 1 in-list of root node 0 / 1, 2 / 3 out-list of
     // root node 0 / 1, -1 none
     int side = -1;
-    if (EVX_ROOT_BOUND && S.kr() >= 3 && !(S.qf & kQNoBound)) {
+    if (EVX_ROOT_BOUND && S.kr() >= 3 && !(S.fl() & kQNoBound)) {
       const int wl = sm.q.plan.info[S.kr() - 2];
       const int a = plan_a(wl), b = plan_b(wl);
       side = b <= 1 ? b : (a <= 1 ? 2 + a : -1);
@@ -1295,7 +1310,7 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
       if (K > 2) sm.slice[lane] = (1 << (16 + sh)) | (lane & ((1 << sh) - 1));
       const bool has = lane < n;
       __syncwarp();
-      if (!ENUM && S.kr() == 2 && (S.qf & kQInlineLast)) {
+      if (!ENUM && S.kr() == 2 && (S.fl() & kQInlineLast)) {
         // the only searched edge closes on the root's endpoints
         if (has) {
           const int4 rt = sm.root[lane];
@@ -1325,7 +1340,7 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
 
 // The shared-memory attribute belongs to the function on the current
 // device, so it is set once per device (bit d of the mask: device d).
-template <int K, bool ENUM, bool EXACT, bool PS, bool CS>
+template <int K, bool ENUM, int TAIL, bool PS, bool CS>
 int setup_k() {
   static std::atomic<unsigned long long> done{0ull};
   int dev = 0;
@@ -1333,11 +1348,11 @@ int setup_k() {
   if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
   const unsigned long long bit = dev < 64 ? (1ull << dev) : 0ull;
   if (bit && (done.load(std::memory_order_acquire) & bit)) return 0;
-  e = cudaFuncSetAttribute(search_kernel<K, ENUM, EXACT, PS, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(search_kernel<K, ENUM, TAIL, PS, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)(kWarps * sizeof(WarpSmem<K>)));
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute");
 #ifdef EVX_CARVEOUT
-  e = cudaFuncSetAttribute(search_kernel<K, ENUM, EXACT, PS, CS>, cudaFuncAttributePreferredSharedMemoryCarveout,
+  e = cudaFuncSetAttribute(search_kernel<K, ENUM, TAIL, PS, CS>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            EVX_CARVEOUT);
   if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(carveout)");
 #endif
@@ -1345,20 +1360,20 @@ int setup_k() {
   return 0;
 }
 
-template <int K, bool ENUM, bool EXACT, bool PS, bool CS>
+template <int K, bool ENUM, int TAIL, bool PS, bool CS>
 int launch_k(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, const EnumArgs &ea, int grid,
              cudaStream_t s) {
-  int rc = setup_k<K, ENUM, EXACT, PS, CS>();
+  int rc = setup_k<K, ENUM, TAIL, PS, CS>();
   if (rc) return rc;
-  search_kernel<K, ENUM, EXACT, PS, CS><<<grid, kBlock, kWarps * sizeof(WarpSmem<K>), s>>>(g, q0, la, ea);
+  search_kernel<K, ENUM, TAIL, PS, CS><<<grid, kBlock, kWarps * sizeof(WarpSmem<K>), s>>>(g, q0, la, ea);
   return 0;
 }
 
-template <int K, bool ENUM, bool EXACT, bool PS, bool CS>
+template <int K, bool ENUM, int TAIL, bool PS, bool CS>
 int occ_k(int *bps) {
-  int rc = setup_k<K, ENUM, EXACT, PS, CS>();
+  int rc = setup_k<K, ENUM, TAIL, PS, CS>();
   if (rc) return rc;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, search_kernel<K, ENUM, EXACT, PS, CS>, kBlock,
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(bps, search_kernel<K, ENUM, TAIL, PS, CS>, kBlock,
                                                                 kWarps * sizeof(WarpSmem<K>));
   return e == cudaSuccess ? 0 : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
 }
@@ -1380,16 +1395,29 @@ QueryDesc single_query(const MotifPlan &plan, const SearchArgs &args) {
 
 }  // namespace
 
-// single-query launches: exact motif size, count or enumerate, with or
-// without the pair-run walk (PS: compiled out where no level needs it), and
-// the constrained variant (CS: node / edge predicates and temporal gaps,
-// always with the walk)
-#define EVX_K_CASE(FN, KK, ...)                                                      \
-  case KK:                                                                           \
-    if (cs) return enumerate ? FN<KK, true, true, true, true>(__VA_ARGS__)            \
-                             : FN<KK, false, true, true, true>(__VA_ARGS__);          \
-    if (enumerate) return ps ? FN<KK, true, true, true, false>(__VA_ARGS__) : FN<KK, true, true, false, false>(__VA_ARGS__); \
-    return ps ? FN<KK, false, true, true, false>(__VA_ARGS__) : FN<KK, false, true, false, false>(__VA_ARGS__);
+// The kernels: exact motif size; count or enumerate; with or without the
+// pair-run walk (PS: compiled out where no level needs it); the constrained
+// variant (CS: node / edge predicates and temporal gaps, always with the walk);
+// and, to count three to five edges, one per way of counting the last edge.
+#define EVX_TAIL_CASE(FN, KK, T, ...) \
+  case T: return ps ? FN<KK, false, T, true, false>(__VA_ARGS__) : FN<KK, false, T, false, false>(__VA_ARGS__);
+#define EVX_K_CASE(FN, KK, ...)                                                       \
+  case KK:                                                                            \
+    if (cs) return enumerate ? FN<KK, true, kTailAny, true, true>(__VA_ARGS__)        \
+                             : FN<KK, false, kTailAny, true, true>(__VA_ARGS__);      \
+    if (enumerate) return ps ? FN<KK, true, kTailAny, true, false>(__VA_ARGS__)       \
+                             : FN<KK, true, kTailAny, false, false>(__VA_ARGS__);     \
+    if constexpr (KK >= 3 && KK <= 5) {                                               \
+      switch (tail) {                                                                 \
+        EVX_TAIL_CASE(FN, KK, kQInlineLast, __VA_ARGS__)                              \
+        EVX_TAIL_CASE(FN, KK, kQSamePair, __VA_ARGS__)                                \
+        EVX_TAIL_CASE(FN, KK, kQRevPair, __VA_ARGS__)                                 \
+        EVX_TAIL_CASE(FN, KK, kQPairHash, __VA_ARGS__)                                \
+        EVX_TAIL_CASE(FN, KK, kQNewArith, __VA_ARGS__)                                \
+        default: break;                                                               \
+      }                                                                               \
+    }                                                                                 \
+    return ps ? FN<KK, false, kTailAny, true, false>(__VA_ARGS__) : FN<KK, false, kTailAny, false, false>(__VA_ARGS__);
 #define EVX_K_DISPATCH(FN, ...)                                        \
   switch (k) {                                                         \
     EVX_K_CASE(FN, 2, __VA_ARGS__)                                     \
@@ -1459,10 +1487,11 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
   const bool ps = plan_pair_scan(plan, q0.flags, enumerate);
   la.cons = args.cons;
   const bool cs = cons_any(args.cons);
+  const int tail = q0.flags & kTailFlags;
   EVX_K_DISPATCH(launch_k, g, q0, la, ea, grid, stream)
 }
 
-int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, bool ps, int grid,
+int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, int tail, bool ps, int grid,
                  cudaStream_t stream) {
   const bool enumerate = false, cs = false;
   EnumArgs ea;
@@ -1470,14 +1499,21 @@ int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, 
   EVX_K_DISPATCH(launch_k, g, q0, la, ea, grid, stream)
 }
 
-int search_occupancy(int k, bool enumerate, bool ps, bool cs, int block, int *blocks_per_sm) {
+int search_occupancy(int k, int qflags, bool enumerate, bool ps, bool cs, int block, int *blocks_per_sm) {
   (void)block;
+  const int tail = qflags & kTailFlags;
   EVX_K_DISPATCH(occ_k, blocks_per_sm)
 }
 
-int table_occupancy(int k, bool ps, int *blocks_per_sm) {
+int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm) {
   const bool enumerate = false, cs = false;
   EVX_K_DISPATCH(occ_k, blocks_per_sm)
+}
+
+int tail_of(int k, int qflags) {
+  const int t = qflags & kTailFlags;
+  const bool one = t == kQInlineLast || t == kQSamePair || t == kQRevPair || t == kQPairHash || t == kQNewArith;
+  return k >= 3 && k <= 5 && one ? t : kTailAny;
 }
 
 int search_block_size() { return kBlock; }
