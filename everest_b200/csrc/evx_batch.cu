@@ -69,8 +69,9 @@ struct evx_batch {
 namespace {
 
 // one work-queue cursor word per launch: motif sizes x ways of counting the
-// last edge (five, and the kernel that holds all)
-constexpr int kCursors = kSizes * 6;
+// last edge (five, with and without strict timestamps, and the kernel that
+// holds all)
+constexpr int kCursors = kSizes * 11;
 // a launch's group of the table: {k, first table position, queries, tiles,
 // grid, pair-run walk (0/1), roots per tile, way of counting the last edge}
 constexpr int kGroupWords = 8;

@@ -106,9 +106,9 @@ constexpr int kScanWide = EVX_SCAN_WIDE;
 #define EVX_ROOT_PACK 1
 #endif
 
-// How a kernel counts the last edge: its kQ* bit where that is compiled in
-// (count mode, no strict timestamps, no constraints), kTailAny where the
-// query's flags say (everything else).  A kernel that holds every way spills
+// How a kernel counts the last edge: its kQ* bit, with kQStrict or not, where
+// that is compiled in (count mode, no constraints), kTailAny where the query's
+// flags say (everything else).  A kernel that holds every way spills
 // (196 bytes of stores for 3 edges, 0 to 88 with one way), and its dead paths
 // cost issue slots: the 36 three-edge queries on 7.8M edges 37.2 -> 30.2 ms.
 constexpr int kTailFlags = kQStrict | kQInlineLast | kQSamePair | kQRevPair | kQPairHash | kQPairDir | kQNewArith;
@@ -1399,8 +1399,11 @@ QueryDesc single_query(const MotifPlan &plan, const SearchArgs &args) {
 // pair-run walk (PS: compiled out where no level needs it); the constrained
 // variant (CS: node / edge predicates and temporal gaps, always with the walk);
 // and, to count three to five edges, one per way of counting the last edge.
-#define EVX_TAIL_CASE(FN, KK, T, ...) \
-  case T: return ps ? FN<KK, false, T, true, false>(__VA_ARGS__) : FN<KK, false, T, false, false>(__VA_ARGS__);
+#define EVX_TAIL_CASE(FN, KK, T, ...)                                                 \
+  case T: return ps ? FN<KK, false, T, true, false>(__VA_ARGS__) : FN<KK, false, T, false, false>(__VA_ARGS__); \
+  case T | kQStrict:                                                                  \
+    return ps ? FN<KK, false, T | kQStrict, true, false>(__VA_ARGS__)                 \
+              : FN<KK, false, T | kQStrict, false, false>(__VA_ARGS__);
 #define EVX_K_CASE(FN, KK, ...)                                                       \
   case KK:                                                                            \
     if (cs) return enumerate ? FN<KK, true, kTailAny, true, true>(__VA_ARGS__)        \
@@ -1511,8 +1514,9 @@ int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm) {
 }
 
 int tail_of(int k, int qflags) {
-  const int t = qflags & kTailFlags;
-  const bool one = t == kQInlineLast || t == kQSamePair || t == kQRevPair || t == kQPairHash || t == kQNewArith;
+  const int t = qflags & kTailFlags, way = t & ~kQStrict;
+  const bool one =
+      way == kQInlineLast || way == kQSamePair || way == kQRevPair || way == kQPairHash || way == kQNewArith;
   return k >= 3 && k <= 5 && one ? t : kTailAny;
 }
 
