@@ -138,9 +138,9 @@ struct evx_worker {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   int num_sms = 148;
-  // small device state (u64 words): [0] count, [1] int cursor + int stop, [2] work meter
-  unsigned long long *state_d = nullptr;
-  unsigned long long *count_h = nullptr;  // pinned
+  WorkerState *state_d = nullptr;
+  bool state_clean = true;                // all zero once the stream's work is done
+  unsigned long long *count_h = nullptr;  // pinned: count, meter
   int *rows_d = nullptr;
   int64_t rows_cap = 0;  // allocated rows
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -386,8 +386,8 @@ int evx_worker_create(int device, void *stream, evx_worker **out) {
     e = cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking);
     w->own_stream = true;
   }
-  if (e == cudaSuccess) e = cudaMalloc(&w->state_d, 64);
-  if (e == cudaSuccess) e = cudaMemset(w->state_d, 0, 64);
+  if (e == cudaSuccess) e = cudaMalloc(&w->state_d, sizeof(WorkerState));
+  if (e == cudaSuccess) e = cudaMemset(w->state_d, 0, sizeof(WorkerState));
   if (e == cudaSuccess) e = cudaMallocHost(&w->count_h, 2 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
@@ -500,11 +500,13 @@ int evx_worker_take(evx_worker *w, const evx_graph *gh, int k, const int *mu, co
   a.exact_total = (flags & EVX_FLAG_EXACT_TOTAL) ? 1 : 0;
   a.cap = enum_cap;
   a.rows = w->rows_d;
-  a.count = w->state_d;
-  a.cursor = reinterpret_cast<int *>(w->state_d + 1);
-  a.stop = reinterpret_cast<int *>(w->state_d + 1) + 1;
+  a.count = &w->state_d->count;
+  a.cursor = &w->state_d->cursor;
+  a.stop = &w->state_d->stop;
   a.limit = (unsigned long long)w->limit;
-  a.meter = w->state_d + 2;
+  a.meter = &w->state_d->meter;
+  a.state = w->state_d;
+  a.out = w->count_h;
   w->enum_cap = enum_cap;
   w->cons_active = false;
   w->has_job = true;
@@ -656,9 +658,9 @@ int evx_worker_take_constrained(evx_worker *w, const evx_graph *gh, int k, const
   cs.node_ok = c->node_mode ? w->node_ok_d : nullptr;
   cs.edge_ok = c->has_edge ? w->edge_ok_d : nullptr;
   cs.edge_feat = g.edge_feat;
-  cs.count = w->state_d;
-  cs.cursor = reinterpret_cast<int *>(w->state_d + 1);
-  cs.stop = reinterpret_cast<int *>(w->state_d + 1) + 1;
+  cs.count = &w->state_d->count;
+  cs.cursor = &w->state_d->cursor;
+  cs.stop = &w->state_d->stop;
   cs.rows = w->rows_d;
   cs.cap = enum_cap;
   w->view = g.view();
@@ -673,11 +675,8 @@ int evx_worker_take_constrained(evx_worker *w, const evx_graph *gh, int k, const
 }
 
 namespace evx {
-__global__ void reset_state_kernel(unsigned long long *count, int *cursor, int *stop, int beg) {
-  *count = 0ull;
-  *cursor = beg;  // the search's work queue: next unclaimed root tile
-  *stop = 0;
-  count[2] = 0ull;  // work meter
+__global__ void reset_state_kernel(WorkerState *s, int beg) {
+  *s = WorkerState{0ull, beg, 0, 0ull, 0u};
 }
 }  // namespace evx
 
@@ -694,7 +693,8 @@ static int launch_constrained_job(evx_worker *w) {
   const int grid = bps * w->num_sms;
   if ((int64_t)c.root_end + (int64_t)grid * cons_block() >= (int64_t)INT_MAX)
     return fail(EVX_ERR_OVERFLOW, "root cursor would overflow int32");
-  reset_state_kernel<<<1, 1, 0, w->stream>>>(c.count, c.cursor, c.stop, c.root_beg);
+  reset_state_kernel<<<1, 1, 0, w->stream>>>(w->state_d, c.root_beg);
+  w->state_clean = false;
   EVX_CUDA(cudaGetLastError());
   EVX_CUDA(cudaEventRecord(w->ev0, w->stream));
   int launches = 1;
@@ -730,22 +730,29 @@ int evx_worker_launch(evx_worker *w) {
   if ((int64_t)a.root_end + warps * (int64_t)a.roots_per_fetch >= (int64_t)INT_MAX)
     return fail(EVX_ERR_OVERFLOW, "root cursor would overflow int32");
   if (w->cons_active) return launch_constrained_job(w);
-  reset_state_kernel<<<1, 1, 0, w->stream>>>(a.count, a.cursor, a.stop, 0);
-  EVX_CUDA(cudaGetLastError());
+  // (a search clears the state it leaves; other jobs and failed launches do not)
+  int launches = 0;
+  if (!w->state_clean) {
+    reset_state_kernel<<<1, 1, 0, w->stream>>>(w->state_d, 0);
+    EVX_CUDA(cudaGetLastError());
+    launches++;
+  }
+  w->state_clean = false;
   EVX_CUDA(cudaEventRecord(w->ev0, w->stream));
-  int launches = 1;
   if (a.root_end > a.root_beg) {
     int rc = launch_search(w->view, w->plan, a, grid, w->block, w->stream);
     if (rc) return rc;
     EVX_CUDA(cudaGetLastError());
     launches++;
+  } else {
+    // no roots: the state's zeros are the result
+    EVX_CUDA(cudaMemcpyAsync(w->count_h, &w->state_d->count, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                             w->stream));
+    EVX_CUDA(cudaMemcpyAsync(w->count_h + 1, &w->state_d->meter, sizeof(unsigned long long),
+                             cudaMemcpyDeviceToHost, w->stream));
   }
   EVX_CUDA(cudaEventRecord(w->ev1, w->stream));
-  EVX_CUDA(cudaMemcpyAsync(w->count_h, a.count, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                           w->stream));
-  if (a.limit)
-    EVX_CUDA(cudaMemcpyAsync(w->count_h + 1, a.meter, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                             w->stream));
+  w->state_clean = true;
   w->last_launches = launches;
   w->launched = true;
   return EVX_OK;

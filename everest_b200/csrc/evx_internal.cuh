@@ -154,6 +154,17 @@ struct ConsArgs {
   int gap[EVX_MAX_MOTIF_EDGES];   // [j-1]: t(e_{j-1}) + gap, not after t(e_0) + delta (j >= 2)
 };
 
+// Device state of a worker's search.  All zero when a launch starts: the last
+// block of a search hands its results to the host and clears it for the next
+// one, which saves a reset kernel and a copy around every search.
+struct WorkerState {
+  unsigned long long count;   // result / enumeration slot counter
+  int cursor;                 // tiles claimed
+  int stop;                   // set when the enumeration cap is reached
+  unsigned long long meter;   // work meter
+  unsigned done;              // blocks that have ended
+};
+
 struct LaunchArgs {
   const QueryDesc *table;     // device table (nq > 1); ignored when nq == 1
   int nq;
@@ -166,6 +177,8 @@ struct LaunchArgs {
   unsigned long long *meter;  // [nq] matches + queued partial matches per query
                               // (maintained only when limit > 0)
   ConsArgs cons;              // single constrained query (the CS kernels); zero otherwise
+  WorkerState *state;         // single query of a worker (null: counts stay where they are)
+  unsigned long long *out;    // [2] host memory: its count and meter
 };
 
 // Search job arguments (one query).
@@ -187,6 +200,8 @@ struct SearchArgs {
   unsigned long long limit;   // work limit (0 = none), count mode only
   unsigned long long *meter;  // [1] matches + queued partial matches (limit > 0)
   ConsArgs cons;              // node / edge predicates and temporal gaps (zero: none)
+  WorkerState *state;         // the worker's state, cleared by the search (null: not)
+  unsigned long long *out;    // [2] host memory: count and meter
 };
 
 // Host-side graph object.

@@ -1336,6 +1336,25 @@ search_kernel(const GraphView g, const __grid_constant__ QueryDesc q0, const Lau
     }
   }
   flush();
+  if (la.state) {
+    // the last block to end hands over the results and clears the state
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      if (atomicAdd(&la.state->done, 1u) == gridDim.x - 1) {
+        __threadfence();
+        volatile WorkerState *st = la.state;
+        volatile unsigned long long *out = la.out;
+        out[0] = st->count;
+        out[1] = st->meter;
+        st->count = 0ull;
+        st->cursor = 0;
+        st->stop = 0;
+        st->meter = 0ull;
+        st->done = 0u;
+      }
+    }
+  }
 }
 
 // The shared-memory attribute belongs to the function on the current
@@ -1487,6 +1506,8 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
   ea.exact_total = args.exact_total;
   ea.stop = args.stop;
   ea.count = args.count;
+  la.state = args.state;
+  la.out = args.out;
   const bool ps = plan_pair_scan(plan, q0.flags, enumerate);
   la.cons = args.cons;
   const bool cs = cons_any(args.cons);
