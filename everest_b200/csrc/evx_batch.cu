@@ -22,6 +22,8 @@
 #include <climits>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -30,7 +32,42 @@
 using namespace evx;
 
 namespace {
-constexpr int kSizes = EVX_MAX_MOTIF_EDGES - 1;  // motif sizes, each a launch of its own
+constexpr int kSizes = EVX_MAX_MOTIF_EDGES - 1;  // motif sizes
+// Streams beside the batch's own (64 mixed queries over 250k-root windows, eight
+// launches: 24.6 ms with one, 20.1 with six; eight drawn batches 2.95 -> 2.46
+// ms).  Creating one takes up to 0.5 ms, so a batch takes them when it first
+// needs them, from those that destroyed batches of the device gave back (at
+// most kSpare are kept), and has them to itself meanwhile.
+constexpr int kSides = 6;
+constexpr size_t kSpare = 4 * kSides;
+std::mutex g_side_mu;
+std::map<int, std::vector<cudaStream_t>> g_spare;  // per device, idle
+
+cudaError_t take_side(int device, cudaStream_t *s) {
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    std::vector<cudaStream_t> &v = g_spare[device];
+    if (!v.empty()) {
+      *s = v.back();
+      v.pop_back();
+      return cudaSuccess;
+    }
+  }
+  return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+
+// (its work is done: the batch's stream has joined it and was waited for)
+void give_side(int device, cudaStream_t s) {
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    std::vector<cudaStream_t> &v = g_spare[device];
+    if (v.size() < kSpare) {
+      v.push_back(s);
+      return;
+    }
+  }
+  cudaStreamDestroy(s);
+}
 }
 
 struct evx_batch {
@@ -46,8 +83,8 @@ struct evx_batch {
   unsigned long long *counts_d = nullptr;  // [max_q] counts, kCursors cursor words, [max_q] work meters
   unsigned long long *counts_h = nullptr;  // pinned [max_q] counts, [max_q] meters
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaStream_t side[kSizes - 1] = {};      // streams of the second and later sizes
-  cudaEvent_t fork = nullptr, join[kSizes - 1] = {};
+  cudaStream_t side[kSides] = {};  // streams beside it, created when first needed
+  cudaEvent_t fork = nullptr, join[kSides] = {};
   // tuning
   int tile_roots = 256, blocks_per_sm = 0, steal_interval = 16, min_split = 2, use_graph = 1;
   unsigned long long limit = 0;  // work limit per query (0 = none)
@@ -95,7 +132,7 @@ int enqueue(evx_batch *b, int nq) {
   for (size_t gi = 0; gi < groups; gi++) {
     const int *gr = &b->groups[gi * kGroupWords];
     const int k = gr[0], beg = gr[1], tiles = gr[3], grid = gr[4];
-    const size_t si = gi ? (gi - 1) % (kSizes - 1) : 0;
+    const size_t si = gi ? (gi - 1) % kSides : 0;
     cudaStream_t s = gi ? b->side[si] : b->stream;
     if (gi) EVX_CUDA(cudaStreamWaitEvent(s, b->fork, 0));
     if (tiles > 0 && !rc) {
@@ -114,7 +151,7 @@ int enqueue(evx_batch *b, int nq) {
     }
   }
   // joined on errors too: a side stream is never left behind in a capture
-  for (size_t i = 0; i + 1 < groups && i < kSizes - 1; i++) {
+  for (size_t i = 0; i + 1 < groups && i < kSides; i++) {
     EVX_CUDA(cudaEventRecord(b->join[i], b->side[i]));
     EVX_CUDA(cudaStreamWaitEvent(b->stream, b->join[i], 0));
   }
@@ -157,11 +194,6 @@ int evx_batch_create(int device, int max_queries, void *stream, evx_batch **out)
   if (e == cudaSuccess) e = cudaMallocHost(&b->counts_h, sizeof(unsigned long long) * 2 * (size_t)max_queries);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&b->ev1);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
-  for (int i = 0; i < kSizes - 1; i++) {
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming);
-  }
   if (e != cudaSuccess) {
     evx_batch_destroy(b);
     return cuda_fail(e, "batch setup");
@@ -183,9 +215,9 @@ int evx_batch_destroy(evx_batch *b) {
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
   if (b->fork) cudaEventDestroy(b->fork);
-  for (int i = 0; i < kSizes - 1; i++) {
+  for (int i = 0; i < kSides; i++) {
     if (b->join[i]) cudaEventDestroy(b->join[i]);
-    if (b->side[i]) cudaStreamDestroy(b->side[i]);
+    if (b->side[i]) give_side(b->device, b->side[i]);
   }
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   delete b;
@@ -307,6 +339,12 @@ int evx_batch_launch(evx_batch *b) {
   }
   if ((int)b->groups.size() / kGroupWords > kCursors)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
+  const int sides = std::min((int)b->groups.size() / kGroupWords - 1, kSides);
+  if (sides > 0 && !b->fork) EVX_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
+  for (int i = 0; i < sides; i++) {
+    if (!b->side[i]) EVX_CUDA(take_side(b->device, &b->side[i]));
+    if (!b->join[i]) EVX_CUDA(cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming));
+  }
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {
     if (!b->exec || b->exec_nq != nq || b->exec_groups != b->groups || b->exec_tile_roots != b->tile_roots ||
