@@ -329,6 +329,7 @@ int evx_batch_launch(evx_batch *b) {
     int tiles = 0;
     for (int i = beg; i < pos; i++) {
       QueryDesc q = b->queries[b->order[i]];
+      if (!b->limit) q.flags = bound_rule(q.plan, q.flags);
       q.tile_beg = tiles;
       const int n = q.root_end - q.root_beg;
       tiles += n > 0 ? (n + tile_roots - 1) / tile_roots : 0;

@@ -129,6 +129,27 @@ int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate) {
   return np;
 }
 
+// The per-root window bound costs a gather and a gallop per root, and saves
+// scans.  Three edges whose last one is counted by range arithmetic have too
+// little left to save: on 7.8M edges, without and with it, 12 fixed-pair
+// queries 4.87 / 5.87 ms, 8 new-node 3.96 / 4.55, 4 same-pair 3.40 / 3.60, 4
+// reverse-pair 3.67 / 3.81; with a pair-table last edge 10.66 / 8.50, with four
+// edges 78 / 62 ms.  (Jobs with a work limit keep the bound: their meter counts
+// the records inside the windows it leaves.)
+int bound_rule(const MotifPlan &plan, int qflags) {
+  const int cheap = kQInlineLast | kQSamePair | kQRevPair | kQNewArith;
+  return plan.k == 3 && (qflags & cheap) ? qflags | kQNoBound : qflags;
+}
+
+// Rounds between rebalances where the caller does not say.  On 7.8M edges, every
+// 4 and every 16 rounds: three edges by range arithmetic 17.8 / 20.5 ms and by
+// the pair table 8.50 / 9.18, four edges 61.8 / 65.2, five no difference; but
+// four edges by the pair table 29.9 / 26.5 (the 4-cycle's windows are short).
+int steal_rule(const MotifPlan &plan, int qflags) {
+  const int arith = kQInlineLast | kQSamePair | kQRevPair | kQNewArith;
+  return plan.k >= 3 && plan.k <= 5 && (qflags & (plan.k == 4 ? arith : arith | kQPairHash)) ? 4 : 16;
+}
+
 }  // namespace evx
 
 using namespace evx;
@@ -154,7 +175,8 @@ struct evx_worker {
   uint64_t last_count = 0;
   uint64_t limit = 0;  // work limit of later jobs (0 = none)
   // tuning
-  int block = 256, blocks_per_sm = 0, roots_per_fetch = 32, steal_interval = 16, min_split = 2;
+  int block = 256, blocks_per_sm = 0, roots_per_fetch = 32, min_split = 2;
+  int steal_interval = -1;  // -1: steal_rule
   int last_launches = 0;
   float last_ms = 0.f;
   // constrained job (evx_worker_take_constrained)
@@ -493,10 +515,13 @@ int evx_worker_take(evx_worker *w, const evx_graph *gh, int k, const int *mu, co
   a.delta = delta;
   a.strict_ts = (flags & EVX_FLAG_STRICT_TS) ? 1 : 0;
   a.roots_per_fetch = w->roots_per_fetch;
-  a.steal_interval = (flags & EVX_FLAG_NO_STEAL) ? 0 : w->steal_interval;
   a.min_split = w->min_split;
   a.enumerate = enum_cap > 0 ? 1 : 0;
   a.tail_flags = tail_mode(plan, flags, enum_cap > 0);
+  if (!w->limit) a.tail_flags = bound_rule(plan, a.tail_flags);
+  a.steal_interval = (flags & EVX_FLAG_NO_STEAL) ? 0
+                     : w->steal_interval >= 0   ? w->steal_interval
+                                                : steal_rule(plan, a.tail_flags);
   a.exact_total = (flags & EVX_FLAG_EXACT_TOTAL) ? 1 : 0;
   a.cap = enum_cap;
   a.rows = w->rows_d;
@@ -644,6 +669,7 @@ int evx_worker_take_constrained(evx_worker *w, const evx_graph *gh, int k, const
     int tf = kQPairScan | (c->has_temporal ? kQNoPrune : 0);
     if (!c->has_edge && !c->has_temporal) tf |= tail_mode(plan, 0, enum_cap > 0) & ~kQNewArith;
     a.tail_flags = tf;
+    if (w->steal_interval < 0) a.steal_interval = 16;
     return EVX_OK;
   }
   cs.plan = plan;

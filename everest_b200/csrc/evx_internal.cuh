@@ -245,6 +245,10 @@ struct DeviceGraph {
 int build_plan(int k, const int *mu, const int *mv, MotifPlan *plan);
 // How a count query counts its last edge (kQInlineLast, kQSamePair or 0).
 int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate);
+// Its flags with the per-root window bound turned off where that is faster.
+int bound_rule(const MotifPlan &plan, int qflags);
+// Rounds between rebalances where the caller does not say.
+int steal_rule(const MotifPlan &plan, int qflags);
 
 // Stream-ordered device allocations from a library-owned pool per device
 // that keeps freed memory mapped (graph re-uploads and pair-index scratch

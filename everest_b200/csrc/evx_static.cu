@@ -83,10 +83,10 @@ int static_query(const DeviceGraph &g, const int *k, const int *mu, const int *m
   a->delta = delta[q];
   a->strict_ts = (flags & EVX_FLAG_STRICT_TS) ? 1 : 0;
   a->roots_per_fetch = 32;
-  a->steal_interval = (flags & EVX_FLAG_NO_STEAL) ? 0 : 16;
   a->min_split = 2;
   a->enumerate = 0;
-  a->tail_flags = tail_mode(*plan, flags, false);
+  a->tail_flags = bound_rule(*plan, tail_mode(*plan, flags, false));
+  a->steal_interval = (flags & EVX_FLAG_NO_STEAL) ? 0 : steal_rule(*plan, a->tail_flags);
   a->count = scratch + q;
   a->cursor = reinterpret_cast<int *>(scratch + EVX_STATIC_MAX_QUERIES + q);
   a->stop = a->cursor + 1;
