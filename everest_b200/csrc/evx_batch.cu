@@ -325,14 +325,15 @@ int evx_batch_launch(evx_batch *b) {
     if (rc) return rc;
     if (b->blocks_per_sm > 0) bps = b->blocks_per_sm;
     if (bps < 1) bps = 1;
-    const int tile_roots = tile_roots_for(k, roots, bps * b->num_sms, b->tile_roots);
+    const long long warps = (long long)bps * b->num_sms * (search_block_size() / 32);
+    const int tile_roots = tile_roots_for(k, roots, pos - beg, warps, b->tile_roots);
+    if (tile_roots == 0) return fail(EVX_ERR_OVERFLOW, "root tiles would overflow int32");
     int tiles = 0;
     for (int i = beg; i < pos; i++) {
       QueryDesc q = b->queries[b->order[i]];
       if (!b->limit) q.flags = bound_rule(q.plan, q.flags);
       q.tile_beg = tiles;
-      const int n = q.root_end - q.root_beg;
-      tiles += n > 0 ? (n + tile_roots - 1) / tile_roots : 0;
+      tiles += (int)tiles_of(q.root_end - q.root_beg, tile_roots);
       b->table_h[i] = q;
     }
     b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots, way});

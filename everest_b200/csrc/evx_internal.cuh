@@ -6,6 +6,7 @@
 #include <string>
 
 #include "../../include/everest_b200.h"
+#include "evx_tiles.h"
 
 namespace evx {
 
@@ -267,9 +268,6 @@ int cuda_fail(cudaError_t e, const char *what);
     if (_e != cudaSuccess) return ::evx::cuda_fail(_e, #call); \
   } while (0)
 
-// Roots per tile of a k-edge launch of `grid` blocks over `roots` roots, `most` at most.
-int tile_roots_for(int k, long long roots, int grid, int most);
-
 // Launch the search for one query (defined in evx_search.cu).
 int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args,
                   int grid, int block, cudaStream_t stream);
@@ -279,6 +277,7 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
 int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, int tail, bool ps, int grid,
                  cudaStream_t stream);
 int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm);
+int search_block_size();  // threads per block of every search kernel
 // The way of counting the last edge that a k-edge kernel with these flags is
 // compiled for (the same negative value for every kernel that holds all ways).
 int tail_of(int k, int qflags);

@@ -42,7 +42,6 @@
 //  * enumeration slots are reserved with one warp-aggregated atomicAdd per
 //    step (the reference issues one atomicAdd per match,
 //    system/tmine/KernelGen.py:505-524).
-#include <algorithm>
 #include <atomic>
 
 #include "evx_internal.cuh"
@@ -1465,25 +1464,6 @@ bool plan_pair_scan(const MotifPlan &plan, int qflags, bool enumerate) {
   return false;
 }
 
-// A tile is what one warp searches alone, so it decides how evenly a launch
-// ends: 64 roots (32 leave batches short after the window bound: the 36
-// three-edge queries on 7.8M edges 37.3 -> 39.8 ms; six five-edge queries on
-// 1.3M edges 2.07 -> 2.09 ms), but 32 for four edges (the 4-cycle on 36M edges
-// 132.9 -> 127.3 ms; 16: 133.2 ms).  A root range too short to give every
-// warp several of those is cut finer.  Up to three edges, down to one tile per
-// warp and no further: a batch costs its latency however few its roots
-// (triangle on 200k edges: 198 us with tiles of 64, 119 with one tile per warp,
-// 163 with four).  More edges, eight tiles per warp of 16 roots or more, since
-// a root's cost varies more (four for five edges and more; 500k roots of the 4-cycle: 2.50 ms with tiles of
-// 64, 1.70 ms with 16, 1.65 ms with 8; four light edges on 321k edges: 149 us
-// with 64, 131 with 19, 179 with 9).
-int tile_roots_for(int k, long long roots, int grid, int most) {
-  const long long per_warp = roots / ((long long)grid * kWarps);
-  const long long t = k <= 3 ? per_warp : std::max(per_warp / (k == 4 ? 8 : 4), std::min(per_warp, 16ll));
-  const long long least = k == 2 ? 32 : 1;  // (two edges: a batch's lanes are not shared, 60 against 64 us on 199k edges)
-  return (int)std::max(least, std::min(t, (long long)std::min(most, k == 4 ? 32 : 64)));
-}
-
 int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args, int grid, int block,
                   cudaStream_t stream) {
   (void)block;
@@ -1494,8 +1474,9 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
   la.table = nullptr;
   la.nq = 1;
   const int n = args.root_end - args.root_beg;
-  la.tile_roots = tile_roots_for(k, n, grid, n);
-  la.total_tiles = n > 0 ? (n + la.tile_roots - 1) / la.tile_roots : 0;
+  la.tile_roots = tile_roots_for(k, n, 1, (long long)grid * kWarps, n);
+  if (la.tile_roots == 0) return fail(EVX_ERR_OVERFLOW, "root tiles would overflow int32");
+  la.total_tiles = (int)tiles_of(n, la.tile_roots);
   la.cursor = args.cursor;
   la.counts = args.count;
   la.limit = args.limit;
