@@ -409,8 +409,11 @@ int evx_worker_create(int device, void *stream, evx_worker **out) {
     w->own_stream = true;
   }
   if (e == cudaSuccess) e = cudaMalloc(&w->state_d, sizeof(WorkerState));
-  if (e == cudaSuccess) e = cudaMemset(w->state_d, 0, sizeof(WorkerState));
+  // (on the worker's stream: the legacy stream's work, a plain cudaMemset among
+  // it, is not ordered before a search on a non-blocking stream)
+  if (e == cudaSuccess) e = cudaMemsetAsync(w->state_d, 0, sizeof(WorkerState), w->stream);
   if (e == cudaSuccess) e = cudaMallocHost(&w->count_h, 2 * sizeof(unsigned long long));
+  if (e == cudaSuccess) w->count_h[0] = w->count_h[1] = 0;
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&w->ev1);
   if (e != cudaSuccess) {
