@@ -24,12 +24,15 @@ OBJ = os.path.join(PKG, "_build")
 INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-NVCC_FLAGS = ["-O3", "--split-compile", "0", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
+NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
               "-Xcompiler", "-fvisibility=hidden", "--expt-relaxed-constexpr"]
 CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-unused-function"]
 
-CORE_CU = ["evx_search.cu", "evx_graph.cu", "evx_pairs.cu", "evx_capi.cu", "evx_batch.cu", "evx_static.cu",
-           "evx_constrained.cu"]
+# (object, source, definitions): the search kernels are compiled once per motif
+# size, the largest first (the longest compile)
+CORE_CU = [(f"evx_search_k{k}", "evx_search.cu", [f"-DEVX_K={k}"]) for k in (5, 8, 4, 7, 3, 6, 2)]
+CORE_CU += [(f, f, []) for f in ("evx_constrained.cu", "evx_pairs.cu", "evx_graph.cu", "evx_capi.cu", "evx_batch.cu",
+                                 "evx_static.cu", "evx_launch.cu")]
 CORE_CC = ["evx_host.cc"]
 
 
@@ -72,14 +75,12 @@ def build(verbose: bool = False, force: bool = False) -> dict:
     hdrs = _headers()
     jobs = []
     objs = []
-    for f in CORE_CU:
+    for name, f, defs in CORE_CU:
         src = os.path.join(CSRC, f)
-        if not os.path.exists(src):
-            continue
-        o = os.path.join(OBJ, f + ".o")
+        o = os.path.join(OBJ, name + ".o")
         objs.append(o)
         if force or _newer(o, [src] + hdrs):
-            jobs.append([_nvcc(), *ARCH, *NVCC_FLAGS, "-I", INCLUDE, "-c", src, "-o", o])
+            jobs.append([_nvcc(), *ARCH, *NVCC_FLAGS, *defs, "-I", INCLUDE, "-c", src, "-o", o])
     for f in CORE_CC:
         src = os.path.join(CSRC, f)
         o = os.path.join(OBJ, f + ".o")

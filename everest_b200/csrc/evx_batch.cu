@@ -325,7 +325,7 @@ int evx_batch_launch(evx_batch *b) {
     if (rc) return rc;
     if (b->blocks_per_sm > 0) bps = b->blocks_per_sm;
     if (bps < 1) bps = 1;
-    const long long warps = (long long)bps * b->num_sms * (search_block_size() / 32);
+    const long long warps = (long long)bps * b->num_sms * (kSearchBlock / 32);
     const int tile_roots = tile_roots_for(k, roots, pos - beg, warps, b->tile_roots);
     if (tile_roots == 0) return fail(EVX_ERR_OVERFLOW, "root tiles would overflow int32");
     int tiles = 0;

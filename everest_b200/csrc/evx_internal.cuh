@@ -124,6 +124,15 @@ constexpr int kQRevPair = 64;    // last edge reverses the previous edge's endpo
 constexpr int kQNewArith = 128;  // a new-node last edge's long windows counted by range arithmetic
 constexpr int kQPairScan = 256;  // a scanned edge between two mapped nodes walks its pair run
 constexpr int kQNoBound = 512;   // no per-root window bound from the last edge's list
+
+// How a kernel counts the last edge: its kQ* bit, with kQStrict or not, where
+// that is compiled in (count mode, no constraints), kTailAny where the query's
+// flags say (everything else).  A kernel that holds every way spills
+// (196 bytes of stores for 3 edges, 0 to 88 with one way), and its dead paths
+// cost issue slots: the 36 three-edge queries on 7.8M edges 37.2 -> 30.2 ms.
+constexpr int kTailFlags = kQStrict | kQInlineLast | kQSamePair | kQRevPair | kQPairHash | kQPairDir | kQNewArith;
+constexpr int kTailAny = -1;
+
 struct QueryDesc {
   MotifPlan plan;
   int root_beg, root_end;  // root edge ids [beg, end)
@@ -268,7 +277,20 @@ int cuda_fail(cudaError_t e, const char *what);
     if (_e != cudaSuccess) return ::evx::cuda_fail(_e, #call); \
   } while (0)
 
-// Launch the search for one query (defined in evx_search.cu).
+constexpr int kSearchBlock = 128;  // threads per block of every search kernel
+
+// Which of a size's kernels a launch takes (evx_search.cu).
+struct SearchKernel {
+  bool enumerate, ps, cs;
+  int tail;
+};
+template <int K>
+int launch_size(const SearchKernel &x, const GraphView &g, const QueryDesc &q0, const LaunchArgs &la,
+                const EnumArgs &ea, int grid, cudaStream_t s);
+template <int K>
+int occupancy_size(const SearchKernel &x, int *blocks_per_sm);
+
+// Launch the search for one query (defined in evx_launch.cu).
 int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args,
                   int grid, int block, cudaStream_t stream);
 // Launch a persistent search over a table of queries (count mode); q0 is
@@ -277,7 +299,6 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
 int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, int tail, bool ps, int grid,
                  cudaStream_t stream);
 int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm);
-int search_block_size();  // threads per block of every search kernel
 // The way of counting the last edge that a k-edge kernel with these flags is
 // compiled for (the same negative value for every kernel that holds all ways).
 int tail_of(int k, int qflags);

@@ -46,12 +46,20 @@
 
 #include "evx_internal.cuh"
 
+// Compiled once per motif size, each to an object and a module of its own: the
+// compiler's output does not depend on how the work is split, the sizes build
+// side by side (34 s, against 139 s in one piece), and a process loads the
+// kernels of the sizes it searches for (its first triangle 37 -> 2.3 ms).
+#ifndef EVX_K
+#error "EVX_K: the motif size that this object searches for"
+#endif
+
 namespace evx {
 namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kCap = 64;        // task slots per buffered level per warp
-constexpr int kBlock = 128;     // threads per block
+constexpr int kBlock = kSearchBlock;
 constexpr int kWarps = kBlock / 32;
 // Records each lane loads per round in a non-last level's scan.
 #ifndef EVX_SCAN_WIDE
@@ -104,14 +112,6 @@ constexpr int kScanWide = EVX_SCAN_WIDE;
 #ifndef EVX_ROOT_PACK
 #define EVX_ROOT_PACK 1
 #endif
-
-// How a kernel counts the last edge: its kQ* bit, with kQStrict or not, where
-// that is compiled in (count mode, no constraints), kTailAny where the query's
-// flags say (everything else).  A kernel that holds every way spills
-// (196 bytes of stores for 3 edges, 0 to 88 with one way), and its dead paths
-// cost issue slots: the 36 three-edge queries on 7.8M edges 37.2 -> 30.2 ms.
-constexpr int kTailFlags = kQStrict | kQInlineLast | kQSamePair | kQRevPair | kQPairHash | kQPairDir | kQNewArith;
-constexpr int kTailAny = -1;
 
 // Resident blocks per SM the register budget aims for (deeper motifs keep more
 // per-level state live).  3 edges: 10 (the 36 queries 30.2 ms; 8: 32.9, 11 and
@@ -1396,132 +1396,44 @@ int occ_k(int *bps) {
   return e == cudaSuccess ? 0 : cuda_fail(e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
 }
 
-// Single-query launch description from the worker's SearchArgs.
-QueryDesc single_query(const MotifPlan &plan, const SearchArgs &args) {
-  QueryDesc q;
-  memset(&q, 0, sizeof(q));
-  q.plan = plan;
-  q.root_beg = args.root_beg;
-  q.root_end = args.root_end;
-  q.delta = args.delta;
-  q.flags = (args.strict_ts ? kQStrict : 0) | args.tail_flags;
-  q.steal_interval = args.steal_interval;
-  q.min_split = args.min_split;
-  q.tile_beg = 0;
-  return q;
-}
-
 }  // namespace
 
-// The kernels: exact motif size; count or enumerate; with or without the
-// pair-run walk (PS: compiled out where no level needs it); the constrained
-// variant (CS: node / edge predicates and temporal gaps, always with the walk);
-// and, to count three to five edges, one per way of counting the last edge.
-#define EVX_TAIL_CASE(FN, KK, T, ...)                                                 \
-  case T: return ps ? FN<KK, false, T, true, false>(__VA_ARGS__) : FN<KK, false, T, false, false>(__VA_ARGS__); \
-  case T | kQStrict:                                                                  \
-    return ps ? FN<KK, false, T | kQStrict, true, false>(__VA_ARGS__)                 \
-              : FN<KK, false, T | kQStrict, false, false>(__VA_ARGS__);
-#define EVX_K_CASE(FN, KK, ...)                                                       \
-  case KK:                                                                            \
-    if (cs) return enumerate ? FN<KK, true, kTailAny, true, true>(__VA_ARGS__)        \
-                             : FN<KK, false, kTailAny, true, true>(__VA_ARGS__);      \
-    if (enumerate) return ps ? FN<KK, true, kTailAny, true, false>(__VA_ARGS__)       \
-                             : FN<KK, true, kTailAny, false, false>(__VA_ARGS__);     \
-    if constexpr (KK >= 3 && KK <= 5) {                                               \
-      switch (tail) {                                                                 \
-        EVX_TAIL_CASE(FN, KK, kQInlineLast, __VA_ARGS__)                              \
-        EVX_TAIL_CASE(FN, KK, kQSamePair, __VA_ARGS__)                                \
-        EVX_TAIL_CASE(FN, KK, kQRevPair, __VA_ARGS__)                                 \
-        EVX_TAIL_CASE(FN, KK, kQPairHash, __VA_ARGS__)                                \
-        EVX_TAIL_CASE(FN, KK, kQNewArith, __VA_ARGS__)                                \
-        default: break;                                                               \
-      }                                                                               \
-    }                                                                                 \
-    return ps ? FN<KK, false, kTailAny, true, false>(__VA_ARGS__) : FN<KK, false, kTailAny, false, false>(__VA_ARGS__);
-#define EVX_K_DISPATCH(FN, ...)                                        \
-  switch (k) {                                                         \
-    EVX_K_CASE(FN, 2, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 3, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 4, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 5, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 6, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 7, __VA_ARGS__)                                     \
-    EVX_K_CASE(FN, 8, __VA_ARGS__)                                     \
-    default: return fail(EVX_ERR_INVALID, "motif edge count out of range");          \
-  }
+// The kernels of this size: count or enumerate; with or without the pair-run
+// walk (PS: compiled out where no level needs it); the constrained variant (CS:
+// node / edge predicates and temporal gaps, always with the walk); and, to count
+// three to five edges, one per way of counting the last edge.
+#define EVX_TAIL_CASE(FN, T, ...)                                                        \
+  case T: return x.ps ? FN<K, false, T, true, false>(__VA_ARGS__) : FN<K, false, T, false, false>(__VA_ARGS__); \
+  case T | kQStrict:                                                                     \
+    return x.ps ? FN<K, false, T | kQStrict, true, false>(__VA_ARGS__)                   \
+                : FN<K, false, T | kQStrict, false, false>(__VA_ARGS__);
+#define EVX_PICK(FN, ...)                                                                \
+  constexpr int K = EVX_K;                                                               \
+  if (x.cs) return x.enumerate ? FN<K, true, kTailAny, true, true>(__VA_ARGS__)          \
+                               : FN<K, false, kTailAny, true, true>(__VA_ARGS__);        \
+  if (x.enumerate) return x.ps ? FN<K, true, kTailAny, true, false>(__VA_ARGS__)         \
+                               : FN<K, true, kTailAny, false, false>(__VA_ARGS__);       \
+  if constexpr (K >= 3 && K <= 5) {                                                      \
+    switch (x.tail) {                                                                    \
+      EVX_TAIL_CASE(FN, kQInlineLast, __VA_ARGS__)                                       \
+      EVX_TAIL_CASE(FN, kQSamePair, __VA_ARGS__)                                         \
+      EVX_TAIL_CASE(FN, kQRevPair, __VA_ARGS__)                                          \
+      EVX_TAIL_CASE(FN, kQPairHash, __VA_ARGS__)                                         \
+      EVX_TAIL_CASE(FN, kQNewArith, __VA_ARGS__)                                         \
+      default: break;                                                                    \
+    }                                                                                    \
+  }                                                                                      \
+  return x.ps ? FN<K, false, kTailAny, true, false>(__VA_ARGS__) : FN<K, false, kTailAny, false, false>(__VA_ARGS__);
 
-// Whether a query walks a pair run at some level: an edge between two nodes
-// mapped before it that is scanned (every level before the last; the last
-// one only when enumerating: a counted closing last edge takes range
-// arithmetic instead).
-bool plan_pair_scan(const MotifPlan &plan, int qflags, bool enumerate) {
-  if (!(qflags & kQPairScan)) return false;
-  for (int l = 0; l <= plan.k - 2; l++) {
-    if (plan_kind(plan.info[l]) != 2) continue;
-    if (l < plan.k - 2 || enumerate) return true;
-  }
-  return false;
+template <>
+int launch_size<EVX_K>(const SearchKernel &x, const GraphView &g, const QueryDesc &q0, const LaunchArgs &la,
+                       const EnumArgs &ea, int grid, cudaStream_t s) {
+  EVX_PICK(launch_k, g, q0, la, ea, grid, s)
 }
 
-int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &args, int grid, int block,
-                  cudaStream_t stream) {
-  (void)block;
-  const int k = plan.k;
-  const bool enumerate = args.enumerate != 0;
-  const QueryDesc q0 = single_query(plan, args);
-  LaunchArgs la{};
-  la.table = nullptr;
-  la.nq = 1;
-  const int n = args.root_end - args.root_beg;
-  la.tile_roots = tile_roots_for(k, n, 1, (long long)grid * kWarps, n);
-  if (la.tile_roots == 0) return fail(EVX_ERR_OVERFLOW, "root tiles would overflow int32");
-  la.total_tiles = (int)tiles_of(n, la.tile_roots);
-  la.cursor = args.cursor;
-  la.counts = args.count;
-  la.limit = args.limit;
-  la.meter = args.meter;
-  EnumArgs ea;
-  ea.rows = args.rows;
-  ea.cap = args.cap;
-  ea.exact_total = args.exact_total;
-  ea.stop = args.stop;
-  ea.count = args.count;
-  la.state = args.state;
-  la.out = args.out;
-  const bool ps = plan_pair_scan(plan, q0.flags, enumerate);
-  la.cons = args.cons;
-  const bool cs = cons_any(args.cons);
-  const int tail = q0.flags & kTailFlags;
-  EVX_K_DISPATCH(launch_k, g, q0, la, ea, grid, stream)
+template <>
+int occupancy_size<EVX_K>(const SearchKernel &x, int *blocks_per_sm) {
+  EVX_PICK(occ_k, blocks_per_sm)
 }
-
-int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, int tail, bool ps, int grid,
-                 cudaStream_t stream) {
-  const bool enumerate = false, cs = false;
-  EnumArgs ea;
-  memset(&ea, 0, sizeof(ea));
-  EVX_K_DISPATCH(launch_k, g, q0, la, ea, grid, stream)
-}
-
-int search_occupancy(int k, int qflags, bool enumerate, bool ps, bool cs, int block, int *blocks_per_sm) {
-  (void)block;
-  const int tail = qflags & kTailFlags;
-  EVX_K_DISPATCH(occ_k, blocks_per_sm)
-}
-
-int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm) {
-  const bool enumerate = false, cs = false;
-  EVX_K_DISPATCH(occ_k, blocks_per_sm)
-}
-
-int tail_of(int k, int qflags) {
-  const int t = qflags & kTailFlags, way = t & ~kQStrict;
-  const bool one =
-      way == kQInlineLast || way == kQSamePair || way == kQRevPair || way == kQPairHash || way == kQNewArith;
-  return k >= 3 && k <= 5 && one ? t : kTailAny;
-}
-
-int search_block_size() { return kBlock; }
 
 }  // namespace evx
