@@ -274,9 +274,9 @@ static int alloc_graph(int device, int64_t E, int64_t V, evx_graph **out, cudaSt
 }
 
 // Checks and packs the host-format arrays on the device; *scratch (for
-// finish_graph) holds the time range, the in-list flag and the list nodes.
+// finish_graph) holds the time range, the list flags and the list nodes.
 static ListScratch list_scratch(const DeviceGraph &g, int *scratch) {
-  return ListScratch{scratch + 32, scratch + 32 + g.num_edges, scratch + 2};
+  return ListScratch{scratch + 32, scratch + 32 + g.num_edges, scratch + 2, scratch + 3};
 }
 
 static int start_graph(evx_graph *h, const int *eg_d, const int *out_v_d, const int *in_v_d, const int *out_r_d,

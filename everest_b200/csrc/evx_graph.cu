@@ -15,7 +15,7 @@
 namespace evx {
 namespace {
 
-// positions: outpos[out_v[p]] = p, inpos[in_v[p]] = p
+// positions: outpos[out_v[p]] = p, inpos[in_v[p]] = p (-1 before)
 __global__ void scatter_pos_kernel(const int *__restrict__ out_v, const int *__restrict__ in_v,
                                    int *__restrict__ outpos, int *__restrict__ inpos, int n) {
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
@@ -24,13 +24,20 @@ __global__ void scatter_pos_kernel(const int *__restrict__ out_v, const int *__r
   }
 }
 
+// The packed edges.  *lost is set when a list does not hold every edge (each
+// has E entries, so one is then named twice): the arrays that the lists fill
+// edge by edge would keep gaps, which a search would take for list positions.
 __global__ void pack_edges_kernel(const int *__restrict__ eg, const int *__restrict__ euid_in,
-                                  const int *__restrict__ outpos, int4 *__restrict__ edges,
-                                  int *__restrict__ euid, int n) {
+                                  const int *__restrict__ outpos, const int *__restrict__ inpos,
+                                  int4 *__restrict__ edges, int *__restrict__ euid, int *lost, int n) {
+  bool bad = false;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    edges[i] = make_int4(eg[3 * i], eg[3 * i + 1], eg[3 * i + 2], outpos[i]);
+    const int at = outpos[i];
+    edges[i] = make_int4(eg[3 * i], eg[3 * i + 1], eg[3 * i + 2], at);
     euid[i] = euid_in ? euid_in[i] : i;
+    bad |= at < 0 || inpos[i] < 0;
   }
+  if (bad) *lost = 1;
 }
 
 // Neighbour signatures: one bit per neighbour (sig_bit) in the node's word.
@@ -130,8 +137,10 @@ int pack_graph(DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *i
   if (E > 0) {
     int *outpos = nullptr;  // edges[].w, staged
     EVX_CUDA(dev_alloc((void **)&outpos, sizeof(int) * (size_t)E, g.device, s));
+    EVX_CUDA(cudaMemsetAsync(outpos, 0xff, sizeof(int) * (size_t)E, s));
+    EVX_CUDA(cudaMemsetAsync(g.inpos, 0xff, sizeof(int) * (size_t)E, s));
     scatter_pos_kernel<<<grid, block, 0, s>>>(out_v_d, in_v_d, outpos, g.inpos, (int)E);
-    pack_edges_kernel<<<grid, block, 0, s>>>(eg_d, euid_d, outpos, g.edges, g.euid, (int)E);
+    pack_edges_kernel<<<grid, block, 0, s>>>(eg_d, euid_d, outpos, g.inpos, g.edges, g.euid, lists.lost, (int)E);
     pack_rec_kernel<<<grid, block, 0, s>>>(out_v_d, in_v_d, g.edges, g.inpos, g.node_rng, g.out_rec,
                                            g.in_rec, g.sig_out, g.sig_in, lists, (int)E);
     dev_free(outpos, s);
@@ -163,7 +172,7 @@ int validate_graph(int device, int64_t E, int64_t V, const int *eg_d, const int 
 }
 
 int graph_t_range(DeviceGraph &g, int *scratch_d, bool *in_grouped, cudaStream_t s) {
-  int h[3] = {0, 0, 0};
+  int h[4] = {0, 0, 0, 0};
   t_range_init_kernel<<<1, 1, 0, s>>>(scratch_d);
   if (g.num_edges > 0) {
     int sms = 148;
@@ -173,6 +182,7 @@ int graph_t_range(DeviceGraph &g, int *scratch_d, bool *in_grouped, cudaStream_t
   EVX_CUDA(cudaGetLastError());
   EVX_CUDA(cudaMemcpyAsync(h, scratch_d, sizeof(h), cudaMemcpyDeviceToHost, s));
   EVX_CUDA(cudaStreamSynchronize(s));
+  if (h[3]) return fail(EVX_ERR_INVALID, "the out/in lists do not hold every edge once");
   *in_grouped = h[2] == 0;
   g.min_t = g.num_edges ? h[0] : 0;
   g.max_t = g.num_edges ? h[1] : 0;

@@ -343,10 +343,11 @@ int cons_build_masks(const evx_constraints &c, int n, const int *node_feat, int 
                      int E, unsigned short *node_ok, unsigned char *edge_ok, int num_sms, cudaStream_t s);
 
 // What packing leaves for the pair index build: the node of each position of
-// the out- and in-lists, and whether an in-list entry is out of place.
+// the out- and in-lists, whether an in-list entry is out of place, and whether
+// a list lacks an edge.
 struct ListScratch {
   int *out_node, *in_node;  // [E]
-  int *stray;
+  int *stray, *lost;
 };
 
 // Build the pair index (defined in evx_pairs.cu); needs the packed graph.
@@ -359,7 +360,7 @@ int validate_graph(int device, int64_t E, int64_t V, const int *eg_d, const int 
                    const int *out_r_d, const int *in_r_d, cudaStream_t s);
 
 // Build the packed device layout from the uploaded host-format arrays
-// (defined in evx_graph.cu) and fill lists (*lists.stray: zero before).
+// (defined in evx_graph.cu) and fill lists (*lists.stray, *lists.lost: zero before).
 int pack_graph(DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *in_v_d,
                const int *out_r_d, const int *in_r_d, const int *euid_d, const ListScratch &lists, cudaStream_t s);
 
