@@ -22,53 +22,32 @@
 #include <climits>
 #include <cstdint>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <string>
 #include <vector>
 
 #include "evx_internal.cuh"
+#include "evx_sides.h"
 
 using namespace evx;
 
 namespace {
 constexpr int kSizes = EVX_MAX_MOTIF_EDGES - 1;  // motif sizes
-// Streams beside the batch's own (64 mixed queries over 250k-root windows, eight
-// launches: 24.6 ms with one, 20.1 with six; eight drawn batches 2.95 -> 2.46
-// ms).  Creating one takes up to 0.5 ms, so a batch takes them when it first
-// needs them, from those that destroyed batches of the device gave back (at
-// most kSpare are kept), and has them to itself meanwhile.
-constexpr int kSides = 6;
-constexpr size_t kSpare = 4 * kSides;
-std::mutex g_side_mu;
-std::map<int, std::vector<cudaStream_t>> g_spare;  // per device, idle
 
-cudaError_t take_side(int device, cudaStream_t *s) {
-  {
-    std::lock_guard<std::mutex> lk(g_side_mu);
-    std::vector<cudaStream_t> &v = g_spare[device];
-    if (!v.empty()) {
-      *s = v.back();
-      v.pop_back();
-      return cudaSuccess;
-    }
-  }
-  return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
-}
-
-// (its work is done: the batch's stream has joined it and was waited for)
-void give_side(int device, cudaStream_t s) {
-  {
-    std::lock_guard<std::mutex> lk(g_side_mu);
-    std::vector<cudaStream_t> &v = g_spare[device];
-    if (v.size() < kSpare) {
-      v.push_back(s);
-      return;
-    }
-  }
-  cudaStreamDestroy(s);
-}
-}
+struct CudaApi {
+  using Error = cudaError_t;
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  static constexpr Error kOk = cudaSuccess;
+  static Error create(Stream *s) { return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking); }
+  static Error destroy(Stream s) { return cudaStreamDestroy(s); }
+  static Error synchronize(Stream s) { return cudaStreamSynchronize(s); }
+  static Error create_event(Event *e) { return cudaEventCreateWithFlags(e, cudaEventDisableTiming); }
+  static Error destroy_event(Event e) { return cudaEventDestroy(e); }
+  static Error record(Event e, Stream s) { return cudaEventRecord(e, s); }
+  static Error wait(Stream s, Event e) { return cudaStreamWaitEvent(s, e, 0); }
+};
+SparePool<CudaApi> g_spare;
+}  // namespace
 
 struct evx_batch {
   int device = 0;
@@ -83,8 +62,7 @@ struct evx_batch {
   unsigned long long *counts_d = nullptr;  // [max_q] counts, kCursors cursor words, [max_q] work meters
   unsigned long long *counts_h = nullptr;  // pinned [max_q] counts, [max_q] meters
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  cudaStream_t side[kSides] = {};  // streams beside it, created when first needed
-  cudaEvent_t fork = nullptr, join[kSides] = {};
+  Sides<CudaApi> sides;  // streams beside it
   // tuning
   int tile_roots = 256, blocks_per_sm = 0, steal_interval = 16, min_split = 2, use_graph = 1;
   unsigned long long limit = 0;  // work limit per query (0 = none)
@@ -125,37 +103,26 @@ int enqueue(evx_batch *b, int nq) {
                            b->stream));
   EVX_CUDA(cudaMemsetAsync(b->counts_d, 0, sizeof(unsigned long long) * (2 * (size_t)b->max_q + kCursors),
                            b->stream));
-  // the first launch runs on the batch's stream, the others beside it
-  const size_t groups = b->groups.size() / kGroupWords;
-  if (groups > 1) EVX_CUDA(cudaEventRecord(b->fork, b->stream));
   int rc = EVX_OK;
-  for (size_t gi = 0; gi < groups; gi++) {
-    const int *gr = &b->groups[gi * kGroupWords];
+  cudaError_t e = b->sides.run(b->stream, (int)(b->groups.size() / kGroupWords), [&](int gi, cudaStream_t s) {
+    const int *gr = &b->groups[(size_t)gi * kGroupWords];
     const int k = gr[0], beg = gr[1], tiles = gr[3], grid = gr[4];
-    const size_t si = gi ? (gi - 1) % kSides : 0;
-    cudaStream_t s = gi ? b->side[si] : b->stream;
-    if (gi) EVX_CUDA(cudaStreamWaitEvent(s, b->fork, 0));
-    if (tiles > 0 && !rc) {
-      LaunchArgs la{};
-      la.table = b->table_d + beg;
-      la.nq = gr[2];
-      la.total_tiles = tiles;
-      la.tile_roots = gr[6];
-      la.cursor = reinterpret_cast<int *>(b->counts_d + b->max_q + gi);
-      la.counts = b->counts_d + beg;
-      la.limit = b->limit;
-      la.meter = meter + beg;
-      rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, gr[7], gr[5] != 0, grid, s);
-      cudaError_t e = cudaGetLastError();
-      if (!rc && e != cudaSuccess) rc = cuda_fail(e, "batch search launch");
-    }
-  }
-  // joined on errors too: a side stream is never left behind in a capture
-  for (size_t i = 0; i + 1 < groups && i < kSides; i++) {
-    EVX_CUDA(cudaEventRecord(b->join[i], b->side[i]));
-    EVX_CUDA(cudaStreamWaitEvent(b->stream, b->join[i], 0));
-  }
+    if (tiles <= 0) return cudaSuccess;
+    LaunchArgs la{};
+    la.table = b->table_d + beg;
+    la.nq = gr[2];
+    la.total_tiles = tiles;
+    la.tile_roots = gr[6];
+    la.cursor = reinterpret_cast<int *>(b->counts_d + b->max_q + gi);
+    la.counts = b->counts_d + beg;
+    la.limit = b->limit;
+    la.meter = meter + beg;
+    rc = launch_table(b->graph->g.view(), b->table_h[beg], la, k, gr[7], gr[5] != 0, grid, s);
+    const cudaError_t le = cudaGetLastError();
+    return rc && le == cudaSuccess ? cudaErrorLaunchFailure : le;
+  });
   if (rc) return rc;
+  if (e != cudaSuccess) return cuda_fail(e, "batch search launch");
   EVX_CUDA(cudaMemcpyAsync(b->counts_h, b->counts_d, sizeof(unsigned long long) * (size_t)nq,
                            cudaMemcpyDeviceToHost, b->stream));
   if (b->limit)
@@ -208,17 +175,13 @@ int evx_batch_destroy(evx_batch *b) {
   cudaSetDevice(b->device);
   if (b->stream) cudaStreamSynchronize(b->stream);
   drop_exec(b);
+  b->sides.drop(g_spare, b->device);
   cudaFree(b->table_d);
   cudaFree(b->counts_d);
   if (b->table_h) cudaFreeHost(b->table_h);
   if (b->counts_h) cudaFreeHost(b->counts_h);
   if (b->ev0) cudaEventDestroy(b->ev0);
   if (b->ev1) cudaEventDestroy(b->ev1);
-  if (b->fork) cudaEventDestroy(b->fork);
-  for (int i = 0; i < kSides; i++) {
-    if (b->join[i]) cudaEventDestroy(b->join[i]);
-    if (b->side[i]) give_side(b->device, b->side[i]);
-  }
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   delete b;
   return EVX_OK;
@@ -341,12 +304,7 @@ int evx_batch_launch(evx_batch *b) {
   }
   if ((int)b->groups.size() / kGroupWords > kCursors)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
-  const int sides = std::min((int)b->groups.size() / kGroupWords - 1, kSides);
-  if (sides > 0 && !b->fork) EVX_CUDA(cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming));
-  for (int i = 0; i < sides; i++) {
-    if (!b->side[i]) EVX_CUDA(take_side(b->device, &b->side[i]));
-    if (!b->join[i]) EVX_CUDA(cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming));
-  }
+  EVX_CUDA(b->sides.ready(g_spare, b->device, (int)b->groups.size() / kGroupWords));
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {
     if (!b->exec || b->exec_nq != nq || b->exec_groups != b->groups || b->exec_tile_roots != b->tile_roots ||

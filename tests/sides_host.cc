@@ -1,0 +1,91 @@
+// Side streams of a batch (everest_b200/csrc/evx_sides.h) against a runtime
+// that fails at any one of its calls.  Prints "ok" or the first broken rule.
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+#include <set>
+#include <vector>
+
+#include "evx_sides.h"
+
+#define CHECK(c) \
+  do { if (!(c)) { std::printf("line %d: %s (n %d, call %d)\n", __LINE__, #c, g_n, g_fail); std::exit(1); } } while (0)
+
+static int g_n, g_fail, g_calls;
+
+struct Fake {
+  using Error = int;
+  using Stream = int;
+  using Event = int;
+  static constexpr Error kOk = 0;
+  static inline int next = 1;
+  static inline std::map<int, int> work, done;   // per stream: launches made, launches known to have ended
+  static inline std::map<int, std::pair<int, int>> at;  // event -> stream, launches it covers
+  static inline std::set<int> streams, events, forked;
+  static int call() { return ++g_calls == g_fail ? 7 : 0; }
+  static Error create(Stream *s) { if (int e = call()) return e; *s = next++; streams.insert(*s); return 0; }
+  static Error destroy(Stream s) { CHECK(streams.erase(s) == 1); return call(); }
+  static Error synchronize(Stream s) { if (int e = call()) return e; done[s] = work[s]; return 0; }
+  static Error create_event(Event *v) { if (int e = call()) return e; *v = next++; events.insert(*v); return 0; }
+  static Error destroy_event(Event v) { CHECK(events.erase(v) == 1); return call(); }
+  static Error record(Event v, Stream s) { if (int e = call()) return e; at[v] = {s, work[s]}; return 0; }
+  static Error wait(Stream s, Event v) {
+    if (int e = call()) return e;
+    CHECK(at.count(v));
+    if (at[v].first == kOwn) forked.insert(s);
+    if (s == kOwn) done[at[v].first] = at[v].second;
+    return 0;
+  }
+  static constexpr int kOwn = -1;
+};
+
+int main() {
+  for (g_n = 1; g_n <= 15; g_n++) {
+    int last = 0;
+    for (g_fail = 0; g_fail <= last; g_fail++) {
+      evx::SparePool<Fake> pool;
+      evx::Sides<Fake> s;
+      bool failed = false;
+      g_calls = 0;
+      for (int round = 0; round < 2; round++) {
+        Fake::forked.clear();
+        if (s.ready(pool, 0, g_n)) { failed = true; continue; }
+        for (int x : Fake::streams) CHECK(Fake::work[x] == Fake::done[x]);  // nothing is taken busy
+        int ran = 0;
+        const int e = s.run(Fake::kOwn, g_n, [&](int i, int st) {
+          CHECK(i == ran);
+          ran++;
+          CHECK(i == 0 ? st == Fake::kOwn : Fake::forked.count(st) == 1);
+          Fake::work[st]++;
+          return Fake::call();
+        });
+        CHECK(e || ran == g_n);
+        if (e) failed = true;
+        for (int x : Fake::streams) CHECK(Fake::work[x] == Fake::done[x] || s.astray);
+      }
+      CHECK(!failed == (g_fail == 0 || g_calls < g_fail));  // every failure is reported
+      s.drop(pool, 0);
+      if (g_fail == 0) last = g_calls;
+      CHECK(Fake::events.empty());
+      // what the pool hands out is idle
+      const int mark = Fake::next;
+      for (int i = 0; i < evx::kSides; i++) {
+        int x = 0;
+        if (pool.take(0, &x)) continue;
+        CHECK(x >= mark || Fake::work[x] == Fake::done[x]);
+        Fake::destroy(x);
+      }
+      CHECK(Fake::streams.empty());
+    }
+  }
+  // a device's idle streams are bounded, and stay with their device
+  evx::SparePool<Fake> pool;
+  g_fail = 0;
+  std::vector<int> got;
+  for (int i = 0; i < 100; i++) { int x; Fake::create(&x); got.push_back(x); }
+  for (int x : got) pool.give(1, x);
+  CHECK((int)Fake::streams.size() == evx::SparePool<Fake>::kSpare);
+  int x;
+  CHECK(pool.take(0, &x) == 0 && x > got.back());
+  std::printf("ok\n");
+}
