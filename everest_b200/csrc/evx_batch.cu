@@ -38,7 +38,10 @@ struct CudaApi {
   using Stream = cudaStream_t;
   using Event = cudaEvent_t;
   static constexpr Error kOk = cudaSuccess;
-  static Error create(Stream *s) { return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking); }
+  static Error create(Stream *s, int priority) {
+    return cudaStreamCreateWithPriority(s, cudaStreamNonBlocking, priority);
+  }
+  static Error priority(Stream s, int *p) { return cudaStreamGetPriority(s, p); }
   static Error destroy(Stream s) { return cudaStreamDestroy(s); }
   static Error synchronize(Stream s) { return cudaStreamSynchronize(s); }
   static Error create_event(Event *e) { return cudaEventCreateWithFlags(e, cudaEventDisableTiming); }
@@ -304,7 +307,7 @@ int evx_batch_launch(evx_batch *b) {
   }
   if ((int)b->groups.size() / kGroupWords > kCursors)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
-  EVX_CUDA(b->sides.ready(g_spare, b->device, (int)b->groups.size() / kGroupWords));
+  EVX_CUDA(b->sides.ready(g_spare, b->device, b->stream, (int)b->groups.size() / kGroupWords));
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {
     if (!b->exec || b->exec_nq != nq || b->exec_groups != b->groups || b->exec_tile_roots != b->tile_roots ||

@@ -12,34 +12,34 @@ namespace evx {
 // launches: 24.6 ms with one, 20.1 with six).
 constexpr int kSides = 6;
 
-// Idle streams that destroyed batches gave back: creating one takes up to 0.5
-// ms.  At most kSpare of a device are kept.
+// Idle streams that destroyed batches gave back, of every priority: creating one
+// takes up to 0.5 ms.  At most kSpare of a device are kept.
 template <class Api>
 class SparePool {
  public:
   static constexpr int kSpare = 4 * kSides, kMost = 256;
 
-  typename Api::Error take(int device, typename Api::Stream *s) {
+  typename Api::Error take(int device, int priority, typename Api::Stream *s) {
     {
       std::lock_guard<std::mutex> lk(mu_);
       for (int i = 0; i < n_; i++) {
-        if (spare_[i].device != device) continue;
+        if (spare_[i].device != device || spare_[i].priority != priority) continue;
         *s = spare_[i].stream;
         spare_[i] = spare_[--n_];
         return Api::kOk;
       }
     }
-    return Api::create(s);
+    return Api::create(s, priority);
   }
 
   // (s is idle)
-  void give(int device, typename Api::Stream s) {
+  void give(int device, int priority, typename Api::Stream s) {
     {
       std::lock_guard<std::mutex> lk(mu_);
       int kept = 0;
       for (int i = 0; i < n_; i++) kept += spare_[i].device == device;
       if (kept < kSpare && n_ < kMost) {
-        spare_[n_++] = {device, s};
+        spare_[n_++] = {device, priority, s};
         return;
       }
     }
@@ -48,7 +48,7 @@ class SparePool {
 
  private:
   struct Spare {
-    int device;
+    int device, priority;
     typename Api::Stream stream;
   };
   std::mutex mu_;
@@ -56,7 +56,8 @@ class SparePool {
   int n_ = 0;
 };
 
-// A batch's side streams, taken when first needed and its alone until dropped.
+// A batch's side streams, of its own stream's priority, taken when first needed
+// and its alone until dropped.
 template <class Api>
 struct Sides {
   using Error = typename Api::Error;
@@ -64,14 +65,16 @@ struct Sides {
   using Event = typename Api::Event;
   Stream side[kSides] = {};
   Event fork = {}, join[kSides] = {};
+  int priority = 0;
   bool astray = false;  // a side stream may have work that the batch's stream has not joined
 
   // Make run() of n launches possible (before a capture begins).
-  Error ready(SparePool<Api> &pool, int device, int n) {
+  Error ready(SparePool<Api> &pool, int device, Stream own, int n) {
     Error e = settle();
+    if (e == Api::kOk && n > 1 && !fork) e = Api::priority(own, &priority);
     if (e == Api::kOk && n > 1 && !fork) e = Api::create_event(&fork);
     for (int i = 0; e == Api::kOk && i < kSides && i + 1 < n; i++) {
-      if (!side[i]) e = pool.take(device, &side[i]);
+      if (!side[i]) e = pool.take(device, priority, &side[i]);
       if (e == Api::kOk && !join[i]) e = Api::create_event(&join[i]);
     }
     return e;
@@ -119,7 +122,7 @@ struct Sides {
     for (int i = 0; i < kSides; i++) {
       if (join[i]) Api::destroy_event(join[i]);
       if (side[i] && astray) Api::destroy(side[i]);
-      else if (side[i]) pool.give(device, side[i]);
+      else if (side[i]) pool.give(device, priority, side[i]);
     }
     if (fork) Api::destroy_event(fork);
     *this = Sides();

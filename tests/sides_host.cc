@@ -23,7 +23,16 @@ struct Fake {
   static inline std::map<int, std::pair<int, int>> at;  // event -> stream, launches it covers
   static inline std::set<int> streams, events, forked;
   static int call() { return ++g_calls == g_fail ? 7 : 0; }
-  static Error create(Stream *s) { if (int e = call()) return e; *s = next++; streams.insert(*s); return 0; }
+  static inline std::map<int, int> prio;
+  static Error create(Stream *s, int p) {
+    if (int e = call()) return e;
+    *s = next++;
+    streams.insert(*s);
+    prio[*s] = p;
+    return 0;
+  }
+  static Error priority(Stream, int *p) { if (int e = call()) return e; *p = own_priority; return 0; }
+  static inline int own_priority = 0;
   static Error destroy(Stream s) { CHECK(streams.erase(s) == 1); return call(); }
   static Error synchronize(Stream s) { if (int e = call()) return e; done[s] = work[s]; return 0; }
   static Error create_event(Event *v) { if (int e = call()) return e; *v = next++; events.insert(*v); return 0; }
@@ -45,17 +54,19 @@ int main() {
     for (g_fail = 0; g_fail <= last; g_fail++) {
       evx::SparePool<Fake> pool;
       evx::Sides<Fake> s;
+      Fake::own_priority = -(g_n % 3);
       bool failed = false;
       g_calls = 0;
       for (int round = 0; round < 2; round++) {
         Fake::forked.clear();
-        if (s.ready(pool, 0, g_n)) { failed = true; continue; }
+        if (s.ready(pool, 0, Fake::kOwn, g_n)) { failed = true; continue; }
         for (int x : Fake::streams) CHECK(Fake::work[x] == Fake::done[x]);  // nothing is taken busy
         int ran = 0;
         const int e = s.run(Fake::kOwn, g_n, [&](int i, int st) {
           CHECK(i == ran);
           ran++;
           CHECK(i == 0 ? st == Fake::kOwn : Fake::forked.count(st) == 1);
+          CHECK(i == 0 || Fake::prio[st] == Fake::own_priority);
           Fake::work[st]++;
           return Fake::call();
         });
@@ -71,21 +82,23 @@ int main() {
       const int mark = Fake::next;
       for (int i = 0; i < evx::kSides; i++) {
         int x = 0;
-        if (pool.take(0, &x)) continue;
+        if (pool.take(0, Fake::own_priority, &x)) continue;
         CHECK(x >= mark || Fake::work[x] == Fake::done[x]);
         Fake::destroy(x);
       }
       CHECK(Fake::streams.empty());
     }
   }
-  // a device's idle streams are bounded, and stay with their device
+  // a device's idle streams are bounded, and keep their device and priority
   evx::SparePool<Fake> pool;
   g_fail = 0;
   std::vector<int> got;
-  for (int i = 0; i < 100; i++) { int x; Fake::create(&x); got.push_back(x); }
-  for (int x : got) pool.give(1, x);
+  for (int i = 0; i < 100; i++) { int x; Fake::create(&x, -1); got.push_back(x); }
+  for (int x : got) pool.give(1, -1, x);
   CHECK((int)Fake::streams.size() == evx::SparePool<Fake>::kSpare);
   int x;
-  CHECK(pool.take(0, &x) == 0 && x > got.back());
+  CHECK(pool.take(0, -1, &x) == 0 && x > got.back());
+  CHECK(pool.take(1, 0, &x) == 0 && x > got.back());
+  CHECK(pool.take(1, -1, &x) == 0 && x <= got.back());
   std::printf("ok\n");
 }
