@@ -17,7 +17,9 @@
 // its heaviest roots, whose SMs the next group's blocks then fill, and the
 // heaviest roots start early (the same 64 queries, one size after the other and
 // in the given order: 30.0 ms; side by side, widest first: 23.4 ms; 64 requests
-// over windows of 1000 roots: 0.61 -> 0.45 ms).
+// over windows of 1000 roots: 0.61 -> 0.45 ms).  A batch that the caller gave a
+// number of blocks per SM runs one launch after the other, one per motif size,
+// and so never holds more.
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -100,6 +102,8 @@ void drop_exec(evx_batch *b) {
   b->exec_nq = -1;
 }
 
+int side_streams(const evx_batch *b) { return b->blocks_per_sm > 0 ? 0 : kSides; }
+
 int enqueue(evx_batch *b, int nq) {
   unsigned long long *meter = b->counts_d + b->max_q + kCursors;
   EVX_CUDA(cudaMemcpyAsync(b->table_d, b->table_h, sizeof(QueryDesc) * (size_t)nq, cudaMemcpyHostToDevice,
@@ -107,7 +111,7 @@ int enqueue(evx_batch *b, int nq) {
   EVX_CUDA(cudaMemsetAsync(b->counts_d, 0, sizeof(unsigned long long) * (2 * (size_t)b->max_q + kCursors),
                            b->stream));
   int rc = EVX_OK;
-  cudaError_t e = b->sides.run(b->stream, (int)(b->groups.size() / kGroupWords), [&](int gi, cudaStream_t s) {
+  cudaError_t e = b->sides.run(b->stream, (int)(b->groups.size() / kGroupWords), side_streams(b), [&](int gi, cudaStream_t s) {
     const int *gr = &b->groups[(size_t)gi * kGroupWords];
     const int k = gr[0], beg = gr[1], tiles = gr[3], grid = gr[4];
     if (tiles <= 0) return cudaSuccess;
@@ -265,7 +269,11 @@ int evx_batch_launch(evx_batch *b) {
   // table order: the largest motifs first, and of one launch the widest
   // windows; one group (and one launch) per size and way of counting the last
   // edge
-  const auto tail = [](const QueryDesc &q) { return tail_of(q.plan.k, q.flags); };
+  // (a batch with a bound on its blocks runs its launches one after the other,
+  // so it has one per size: 64 requests over windows of 1000 roots, 4 blocks
+  // per SM, 0.96 ms with one per way and 0.78 with one per size)
+  const bool one = !side_streams(b);
+  const auto tail = [one](const QueryDesc &q) { return one ? kTailAny : tail_of(q.plan.k, q.flags); };
   b->order.resize(nq);
   for (int i = 0; i < nq; i++) b->order[i] = i;
   std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {
@@ -307,7 +315,7 @@ int evx_batch_launch(evx_batch *b) {
   }
   if ((int)b->groups.size() / kGroupWords > kCursors)
     return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
-  EVX_CUDA(b->sides.ready(g_spare, b->device, b->stream, (int)b->groups.size() / kGroupWords));
+  EVX_CUDA(b->sides.ready(g_spare, b->device, b->stream, (int)b->groups.size() / kGroupWords, side_streams(b)));
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {
     if (!b->exec || b->exec_nq != nq || b->exec_groups != b->groups || b->exec_tile_roots != b->tile_roots ||

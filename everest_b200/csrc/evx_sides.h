@@ -68,12 +68,13 @@ struct Sides {
   int priority = 0;
   bool astray = false;  // a side stream may have work that the batch's stream has not joined
 
-  // Make run() of n launches possible (before a capture begins).
-  Error ready(SparePool<Api> &pool, int device, Stream own, int n) {
+  // Make run() of n launches on `sides` streams possible (before a capture begins).
+  Error ready(SparePool<Api> &pool, int device, Stream own, int n, int sides) {
     Error e = settle();
+    if (!sides) return e;
     if (e == Api::kOk && n > 1 && !fork) e = Api::priority(own, &priority);
     if (e == Api::kOk && n > 1 && !fork) e = Api::create_event(&fork);
-    for (int i = 0; e == Api::kOk && i < kSides && i + 1 < n; i++) {
+    for (int i = 0; e == Api::kOk && i < sides && i + 1 < n; i++) {
       if (!side[i]) e = pool.take(device, priority, &side[i]);
       if (e == Api::kOk && !join[i]) e = Api::create_event(&join[i]);
     }
@@ -81,20 +82,21 @@ struct Sides {
   }
 
   // launch(i, stream) for i in [0, n): the first on `own`, the others beside it
-  // and joined to it.  What was forked is joined on an error too, the first
+  // on `sides` streams and joined to it (none: all on `own`, one after the
+  // other).  What was forked is joined on an error too, the first
   // error is returned, and a stream whose join failed is waited for before it
   // is used again or given away.
   template <class F>
-  Error run(Stream own, int n, F launch) {
-    Error e = n > 1 ? Api::record(fork, own) : Api::kOk;
+  Error run(Stream own, int n, int sides, F launch) {
+    Error e = n > 1 && sides ? Api::record(fork, own) : Api::kOk;
     int forked = 0;
     for (int i = 0; e == Api::kOk && i < n; i++) {
-      if (i > forked && forked < kSides) {
+      if (i > forked && forked < sides) {
         e = Api::wait(side[forked], fork);
         if (e != Api::kOk) break;
         forked++;
       }
-      e = launch(i, i ? side[(i - 1) % kSides] : own);
+      e = launch(i, i && sides ? side[(i - 1) % sides] : own);
     }
     for (int i = 0; i < forked; i++) {
       Error j = Api::record(join[i], side[i]);

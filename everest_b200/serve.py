@@ -338,7 +338,7 @@ class Server:
             for r in take:
                 b.add(self.graphs[r.graph], r.mu, r.mv, r.delta, r.beg, r.end, r.flags)
             if self.batch_share < 1.0 and hasattr(b, "set_tuning"):
-                full = 8 if key[1] <= 3 else (6 if key[1] == 4 else 4)  # the kernels' register budgets
+                full = 10 if key[1] <= 3 else (7 if key[1] == 4 else 4)  # the kernels' register budgets
                 b.set_tuning(tile_roots=self.tile_roots, blocks_per_sm=max(1, int(full * self.batch_share)),
                              use_graph=self.use_graph)
             b.launch()

@@ -236,8 +236,10 @@ EVX_API int evx_batch_run(evx_batch *b, uint64_t *counts, int n);
 /* *done = 1 when the launched batch has finished (never blocks). */
 EVX_API int evx_batch_query(evx_batch *b, int *done);
 /* tile_roots (multiple of 32: the most roots of a work-queue tile; short root
- * ranges and larger motifs are cut finer), blocks per SM (0 = occupancy), steal
- * interval, min split, use_graph (capture + replay), reserved. */
+ * ranges and larger motifs are cut finer), blocks per SM (0 = occupancy, and the
+ * launches run side by side; else the most that the batch holds at a time: its
+ * launches, one per motif size, run one after the other), steal interval, min
+ * split, use_graph (capture + replay), reserved. */
 EVX_API int evx_batch_set_tuning(evx_batch *b, int tile_roots, int blocks_per_sm, int steal_interval,
                                  int min_split, int use_graph, int reserved);
 EVX_API int evx_batch_last_stats(evx_batch *b, int *kernel_launches, float *device_ms);

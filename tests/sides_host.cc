@@ -49,7 +49,9 @@ struct Fake {
 };
 
 int main() {
-  for (g_n = 1; g_n <= 15; g_n++) {
+  for (int round = 0; round < 30; round++) {
+    g_n = 1 + round % 15;
+    const int sides = round < 15 ? evx::kSides : 0;
     int last = 0;
     for (g_fail = 0; g_fail <= last; g_fail++) {
       evx::SparePool<Fake> pool;
@@ -57,16 +59,16 @@ int main() {
       Fake::own_priority = -(g_n % 3);
       bool failed = false;
       g_calls = 0;
-      for (int round = 0; round < 2; round++) {
+      for (int pass = 0; pass < 2; pass++) {
         Fake::forked.clear();
-        if (s.ready(pool, 0, Fake::kOwn, g_n)) { failed = true; continue; }
+        if (s.ready(pool, 0, Fake::kOwn, g_n, sides)) { failed = true; continue; }
         for (int x : Fake::streams) CHECK(Fake::work[x] == Fake::done[x]);  // nothing is taken busy
         int ran = 0;
-        const int e = s.run(Fake::kOwn, g_n, [&](int i, int st) {
+        const int e = s.run(Fake::kOwn, g_n, sides, [&](int i, int st) {
           CHECK(i == ran);
           ran++;
-          CHECK(i == 0 ? st == Fake::kOwn : Fake::forked.count(st) == 1);
-          CHECK(i == 0 || Fake::prio[st] == Fake::own_priority);
+          CHECK(i == 0 || !sides ? st == Fake::kOwn : Fake::forked.count(st) == 1);
+          CHECK(st == Fake::kOwn || Fake::prio[st] == Fake::own_priority);
           Fake::work[st]++;
           return Fake::call();
         });
