@@ -28,9 +28,10 @@ from typing import Dict, Optional, Sequence, Tuple
 
 from . import capi
 
-DEFAULT = {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": 0}
+DEFAULT = {"blocks_per_sm": 0, "steal_interval": -1, "min_split": 2, "flags": 0}  # a new worker's
 CANDIDATES = [
     DEFAULT,
+    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": 0},
     {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": 0},
     {"blocks_per_sm": 0, "steal_interval": 64, "min_split": 4, "flags": 0},
     {"blocks_per_sm": 0, "steal_interval": 0, "min_split": 2, "flags": capi.FLAG_NO_STEAL},

@@ -391,8 +391,10 @@ class Worker:
         check(lib().evx_worker_stream(self._h, ctypes.byref(s)))
         return s.value or 0
 
-    def set_tuning(self, block=256, blocks_per_sm=0, roots_per_fetch=32, steal_interval=16,
+    def set_tuning(self, block=256, blocks_per_sm=0, roots_per_fetch=32, steal_interval=-1,
                    min_split=2):
+        """Launch parameters of the jobs taken from now on; the defaults are a
+        new worker's (steal_interval -1: chosen by the query)."""
         check(lib().evx_worker_set_tuning(self._h, block, blocks_per_sm, roots_per_fetch,
                                           steal_interval, min_split))
 

@@ -176,7 +176,7 @@ struct evx_worker {
   uint64_t limit = 0;  // work limit of later jobs (0 = none)
   // tuning
   int block = 256, blocks_per_sm = 0, roots_per_fetch = 32, min_split = 2;
-  int steal_interval = -1;  // -1: steal_rule
+  int steal_interval = -1;  // -1: by steal_rule
   int last_launches = 0;
   float last_ms = 0.f;
   // constrained job (evx_worker_take_constrained)
@@ -451,11 +451,11 @@ int evx_worker_set_tuning(evx_worker *w, int block, int blocks_per_sm, int roots
   if (!w) return fail(EVX_ERR_INVALID, "null worker");
   if (block < 32 || block > 256 || block % 32)
     return fail(EVX_ERR_INVALID, "block must be a multiple of 32 in [32, 256]");
-  if (blocks_per_sm < 0 || roots_per_fetch < 1 || roots_per_fetch > 4096 || steal_interval < 0 ||
+  if (blocks_per_sm < 0 || roots_per_fetch < 1 || roots_per_fetch > 4096 || steal_interval < -1 ||
       min_split < 2)
     return fail(EVX_ERR_INVALID, "bad tuning value");
-  if (steal_interval & (steal_interval - 1))
-    return fail(EVX_ERR_INVALID, "steal_interval must be 0 or a power of two");
+  if (steal_interval > 0 && (steal_interval & (steal_interval - 1)))
+    return fail(EVX_ERR_INVALID, "steal_interval must be -1, 0 or a power of two");
   w->block = block;
   w->blocks_per_sm = blocks_per_sm;
   w->roots_per_fetch = roots_per_fetch;

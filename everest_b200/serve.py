@@ -360,15 +360,15 @@ class Server:
             with self.lock:
                 self.enum_q.popleft()
                 self.enum_reqs[i] = r  # claimed under the lock (see the batches above)
+            if self.enum_blocks_per_sm and hasattr(w, "set_tuning"):  # (before take(), which reads it)
+                busy = bool(self.count_q) or any(x is not None for x in self.batch_reqs)
+                w.set_tuning(block=128, blocks_per_sm=self.enum_blocks_per_sm if busy else 0, roots_per_fetch=32,
+                             steal_interval=-1, min_split=2)
             if r.constraints is not None:
                 w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, r.beg, r.end, r.enum_cap, r.flags,
                        constraints=r.constraints)
             else:
                 w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, r.beg, r.end, r.enum_cap, r.flags)
-            if self.enum_blocks_per_sm and hasattr(w, "set_tuning"):
-                busy = bool(self.count_q) or any(x is not None for x in self.batch_reqs)
-                w.set_tuning(block=128, blocks_per_sm=self.enum_blocks_per_sm if busy else 0, roots_per_fetch=32,
-                             steal_interval=16, min_split=2)
             w.launch()
             self.enum_t0[i] = time.perf_counter()
             progressed = True
@@ -399,11 +399,6 @@ class Server:
                 if job.next_root >= job.end_root:
                     self.heavy_q.popleft()  # every chunk handed out
                 self.heavy_reqs[i] = (job, b0, b1)
-            if r.constraints is not None:
-                w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, b0, b1, r.enum_cap, r.flags,
-                       constraints=r.constraints)
-            else:
-                w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, b0, b1, r.enum_cap, r.flags)
             if hasattr(w, "set_tuning"):
                 # beside other work a heavy chunk takes a fraction of the SMs
                 # (a persistent kernel holds its blocks until it ends); alone
@@ -412,7 +407,12 @@ class Server:
                 busy = bool(self.count_q or self.enum_q) or any(x is not None for x in self.batch_reqs) \
                     or any(x is not None for x in self.enum_reqs)
                 w.set_tuning(block=128, blocks_per_sm=self.heavy_blocks_per_sm if busy else 0,
-                             roots_per_fetch=32, steal_interval=16, min_split=2)
+                             roots_per_fetch=32, steal_interval=-1, min_split=2)
+            if r.constraints is not None:
+                w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, b0, b1, r.enum_cap, r.flags,
+                       constraints=r.constraints)
+            else:
+                w.take(self.graphs[r.graph], r.mu, r.mv, r.delta, b0, b1, r.enum_cap, r.flags)
             w.launch()
             self.heavy_t0[i] = time.perf_counter()
             progressed = True

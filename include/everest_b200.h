@@ -189,8 +189,9 @@ EVX_API int evx_worker_query(evx_worker *w, int *done);
 EVX_API int evx_worker_enum_rows(evx_worker *w, int64_t n, int *rows, int64_t *rows_written);
 
 /* Tuning knobs (autotuner): block size, blocks per SM (0 = occupancy),
- * roots per warp fetch, steal check interval (iterations, 0 = never),
- * minimum range width worth splitting. */
+ * roots per warp fetch, steal check interval (iterations, 0 = never, -1 = by
+ * the query, as a new worker has it; read when a job is taken), minimum range
+ * width worth splitting. */
 EVX_API int evx_worker_set_tuning(evx_worker *w, int block, int blocks_per_sm,
                           int roots_per_fetch, int steal_interval, int min_split);
 

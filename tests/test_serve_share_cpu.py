@@ -27,3 +27,38 @@ def test_batch_share(graph, share, want):  # noqa: F811
         srv.drain(60)
     srv.close()
     assert asked == want
+
+
+def test_slots_are_tuned_before_each_job(graph):  # noqa: F811
+    # a job reads the interval when it is taken: every job of an enumeration
+    # or heavy slot runs by the rule, the first as the later ones
+    be = FakeBackend({"g": graph}, free_bytes=1 << 40)
+    make, calls = be.Worker, {}
+
+    def worker(device):
+        w = make(device)
+        log = calls.setdefault(id(w), [])
+        tune, take = w.set_tuning, w.take
+        w.keep = w  # (the id stays its own)
+
+        def set_tuning(**kw):
+            log.append(kw["steal_interval"])
+            tune(**kw)
+
+        def taken(*a, **kw):
+            log.append("take")
+            take(*a, **kw)
+        w.set_tuning, w.take = set_tuning, taken
+        return w
+    be.Worker = worker
+    srv = serve.Server(max_batch=4, inflight_batches=1, enum_slots=1, mem_reserve=0, backend=be, limit=1, heavy_slots=1)
+    srv.add_graph("g", "g")
+    for _ in range(3):
+        srv.submit("g", [0, 1, 2], [1, 2, 0], 2000, enum_cap=10)
+        srv.submit("g", [0, 1, 2], [1, 2, 0], 3000)
+        srv.drain(60)
+    srv.close()
+    logs = [x for x in calls.values() if x]
+    assert len(logs) == 2  # the enumeration slot's and the heavy slot's
+    for x in logs:
+        assert len(x) >= 6 and x == [-1, "take"] * (len(x) // 2)
