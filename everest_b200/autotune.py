@@ -28,29 +28,37 @@ from typing import Dict, Optional, Sequence, Tuple
 
 from . import capi
 
-DEFAULT = {"blocks_per_sm": 0, "steal_interval": -1, "min_split": 2, "flags": 0}  # a new worker's
+def _cfg(interval: int, flags: int, blocks_per_sm: int = 0, min_split: int = 2) -> dict:
+    return {"blocks_per_sm": blocks_per_sm, "steal_interval": interval, "min_split": min_split, "flags": flags}
+
+
+DEFAULT = _cfg(-1, 0)  # a new worker's: interval and window bound chosen by the query
+# The others say both, so that no two of them are the same search.
+_ON, _OFF = capi.FLAG_ROOT_BOUND, capi.FLAG_NO_ROOT_BOUND
 CANDIDATES = [
     DEFAULT,
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": 0},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": 0},
-    {"blocks_per_sm": 0, "steal_interval": 64, "min_split": 4, "flags": 0},
-    {"blocks_per_sm": 0, "steal_interval": 0, "min_split": 2, "flags": capi.FLAG_NO_STEAL},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_NO_PAIR_INDEX},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_PAIR_DIR},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_PAIR_DIR},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_CLOSING_SCAN},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_CLOSING_SCAN},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_NO_CLOSING_PRUNE},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_NEW_SCAN},
-    {"blocks_per_sm": 4, "steal_interval": 16, "min_split": 2, "flags": 0},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_LIST_SCAN},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_NO_ROOT_BOUND},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_NO_ROOT_BOUND},
-    {"blocks_per_sm": 0, "steal_interval": 64, "min_split": 4, "flags": capi.FLAG_NO_ROOT_BOUND},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2,
-     "flags": capi.FLAG_NO_CLOSING_PRUNE | capi.FLAG_NO_ROOT_BOUND},
-    {"blocks_per_sm": 0, "steal_interval": 4, "min_split": 2, "flags": capi.FLAG_NEW_SCAN | capi.FLAG_NO_ROOT_BOUND},
-    {"blocks_per_sm": 0, "steal_interval": 16, "min_split": 2, "flags": capi.FLAG_PAIR_DIR | capi.FLAG_NO_ROOT_BOUND},
+    _cfg(16, _ON),
+    _cfg(4, _ON),
+    _cfg(64, _ON, min_split=4),
+    _cfg(0, _ON | capi.FLAG_NO_STEAL),
+    _cfg(16, _ON | capi.FLAG_NO_PAIR_INDEX),
+    _cfg(16, _ON | capi.FLAG_PAIR_DIR),
+    _cfg(4, _ON | capi.FLAG_PAIR_DIR),
+    _cfg(16, _ON | capi.FLAG_CLOSING_SCAN),
+    _cfg(4, _ON | capi.FLAG_CLOSING_SCAN),
+    _cfg(4, _ON | capi.FLAG_NO_CLOSING_PRUNE),
+    _cfg(4, _ON | capi.FLAG_NEW_SCAN),
+    _cfg(16, _ON, blocks_per_sm=4),
+    _cfg(16, _ON | capi.FLAG_LIST_SCAN),
+    _cfg(16, _OFF),
+    _cfg(4, _OFF),
+    _cfg(64, _OFF, min_split=4),
+    _cfg(0, _OFF | capi.FLAG_NO_STEAL),
+    _cfg(4, _OFF | capi.FLAG_NO_CLOSING_PRUNE),
+    _cfg(4, _OFF | capi.FLAG_NEW_SCAN),
+    _cfg(16, _OFF | capi.FLAG_PAIR_DIR),
+    _cfg(16, _OFF, blocks_per_sm=4),
+    _cfg(16, _OFF | capi.FLAG_LIST_SCAN),
 ]
 BATCH_TILES = (64, 128, 256, 512)
 

@@ -35,6 +35,7 @@ FLAG_LIST_SCAN = 256
 FLAG_PER_LANE = 512
 FLAG_WARP_SYNC = 1024
 FLAG_NO_ROOT_BOUND = 2048
+FLAG_ROOT_BOUND = 4096
 MAX_MOTIF_EDGES = 8
 
 # every symbol include/everest_b200.h declares

@@ -111,6 +111,7 @@ int build_plan(int k, const int *mu, const int *mv, MotifPlan *plan) {
 int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate) {
   const int np = ((flags & EVX_FLAG_NO_CLOSING_PRUNE) ? kQNoPrune : 0) |
                  ((flags & EVX_FLAG_NO_ROOT_BOUND) ? kQNoBound : 0) |
+                 ((flags & EVX_FLAG_ROOT_BOUND) ? kQKeepBound : 0) |
                  ((flags & (EVX_FLAG_LIST_SCAN | EVX_FLAG_NO_PAIR_INDEX | EVX_FLAG_CLOSING_SCAN)) ? 0 : kQPairScan);
   const int k = plan.k;
   if (enumerate || (flags & EVX_FLAG_NO_PAIR_INDEX) || k < 2) return np;
@@ -138,7 +139,7 @@ int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate) {
 // the records inside the windows it leaves.)
 int bound_rule(const MotifPlan &plan, int qflags) {
   const int cheap = kQInlineLast | kQSamePair | kQRevPair | kQNewArith;
-  return plan.k == 3 && (qflags & cheap) ? qflags | kQNoBound : qflags;
+  return plan.k == 3 && (qflags & cheap) && !(qflags & kQKeepBound) ? qflags | kQNoBound : qflags;
 }
 
 // Rounds between rebalances where the caller does not say.  On 7.8M edges, every

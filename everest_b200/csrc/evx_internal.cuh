@@ -124,6 +124,7 @@ constexpr int kQRevPair = 64;    // last edge reverses the previous edge's endpo
 constexpr int kQNewArith = 128;  // a new-node last edge's long windows counted by range arithmetic
 constexpr int kQPairScan = 256;  // a scanned edge between two mapped nodes walks its pair run
 constexpr int kQNoBound = 512;   // no per-root window bound from the last edge's list
+constexpr int kQKeepBound = 1024;  // host only: that bound whatever bound_rule says
 
 // How a kernel counts the last edge: its kQ* bit, with kQStrict or not, where
 // that is compiled in (count mode, no constraints), kTailAny where the query's
@@ -255,7 +256,8 @@ struct DeviceGraph {
 int build_plan(int k, const int *mu, const int *mv, MotifPlan *plan);
 // How a count query counts its last edge (kQInlineLast, kQSamePair or 0).
 int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate);
-// Its flags with the per-root window bound turned off where that is faster.
+// Its flags with the per-root window bound turned off where that is faster and
+// the caller did not ask for it.
 int bound_rule(const MotifPlan &plan, int qflags);
 // Rounds between rebalances where the caller does not say.
 int steal_rule(const MotifPlan &plan, int qflags);

@@ -67,8 +67,11 @@ extern "C" {
 #define EVX_FLAG_LIST_SCAN 256u
 /* When the last motif edge has a root node as an endpoint, each root's
  * window ends at that node's last entry inside it (a root with none is
- * skipped); this keeps the plain window (same results, for timing). */
+ * skipped), unless the query is one for which the look costs more than it
+ * saves.  NO_ROOT_BOUND keeps the plain window, ROOT_BOUND the bound (same
+ * results, for timing; both: the plain window). */
 #define EVX_FLAG_NO_ROOT_BOUND 2048u
+#define EVX_FLAG_ROOT_BOUND 4096u
 /* evx_worker_take_constrained: a query without anti-edges or a filter (node
  * and edge predicates, temporal gaps) runs on the warp-synchronous search;
  * EVX_FLAG_PER_LANE sends it to the per-lane search instead.
