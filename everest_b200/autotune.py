@@ -60,7 +60,7 @@ CANDIDATES = [
     _cfg(16, _OFF, blocks_per_sm=4),
     _cfg(16, _OFF | capi.FLAG_LIST_SCAN),
 ]
-BATCH_TILES = (64, 128, 256, 512)
+BATCH_TILES = (32, 64)  # (tiles hold 64 roots at most)
 
 
 def graph_key(graph: capi.DeviceGraph) -> str:

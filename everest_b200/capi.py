@@ -475,7 +475,7 @@ class Worker:
 # -------------------------------------------------------------- batches --
 
 class Batch:
-    """Many count queries on one resident graph in one persistent launch."""
+    """Many count queries on one resident graph in a few persistent launches, side by side."""
 
     def __init__(self, device: int = 0, max_queries: int = 1024, stream: Optional[int] = None):
         h = ctypes.c_void_p()
@@ -485,6 +485,8 @@ class Batch:
         self.n = 0
 
     def set_tuning(self, tile_roots=256, blocks_per_sm=0, steal_interval=16, min_split=2, use_graph=True):
+        """tile_roots: the most roots of a tile (above 64, or 32 for four
+        edges, it acts as that); blocks_per_sm: the most the batch holds."""
         check(lib().evx_batch_set_tuning(self._h, tile_roots, blocks_per_sm, steal_interval, min_split,
                                          1 if use_graph else 0, 0))
 

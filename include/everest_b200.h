@@ -219,12 +219,12 @@ EVX_API int evx_worker_set_limit(evx_worker *w, uint64_t max_work);
 
 /* -------------------------------------------------------------- batches --
  * Many count queries against one resident graph in one persistent launch
- * per motif size (no counterpart in the reference, whose batch driver
- * re-generates, re-compiles and re-launches per query,
- * system/batch-query.py:14-20 and system/tmine/frontend.py:135-143).  The
- * root ranges of a size's queries are cut into tiles that form one device
- * work queue.  The launch sequence is captured in a CUDA graph and replayed
- * while the batch keeps its shape. */
+ * per motif size and way of counting the last edge, side by side (no
+ * counterpart in the reference, whose batch driver re-generates, re-compiles
+ * and re-launches per query, system/batch-query.py:14-20 and
+ * system/tmine/frontend.py:135-143).  The root ranges of a launch's queries
+ * are cut into tiles that form one device work queue.  The launch sequence is
+ * captured in a CUDA graph and replayed while the batch keeps its shape. */
 typedef struct evx_batch evx_batch;
 EVX_API int evx_batch_create(int device, int max_queries, void *stream, evx_batch **out);
 EVX_API int evx_batch_destroy(evx_batch *b);
@@ -239,11 +239,12 @@ EVX_API int evx_batch_result(evx_batch *b, uint64_t *counts, int n);
 EVX_API int evx_batch_run(evx_batch *b, uint64_t *counts, int n);
 /* *done = 1 when the launched batch has finished (never blocks). */
 EVX_API int evx_batch_query(evx_batch *b, int *done);
-/* tile_roots (multiple of 32: the most roots of a work-queue tile; short root
- * ranges and larger motifs are cut finer), blocks per SM (0 = occupancy, and the
- * launches run side by side; else the most that the batch holds at a time: its
- * launches, one per motif size, run one after the other), steal interval, min
- * split, use_graph (capture + replay), reserved. */
+/* tile_roots: the most roots of a work-queue tile, a multiple of 32.  Values
+ * above 64 (32 for four edges) act as that, short root ranges are cut finer,
+ * and only a batch of some 2^31 such tiles has larger ones.  blocks_per_sm: 0 =
+ * occupancy, the launches side by side; else the most that the batch holds at
+ * a time (its launches, one per motif size, run one after the other).
+ * steal_interval, min_split, use_graph (capture + replay), reserved. */
 EVX_API int evx_batch_set_tuning(evx_batch *b, int tile_roots, int blocks_per_sm, int steal_interval,
                                  int min_split, int use_graph, int reserved);
 EVX_API int evx_batch_last_stats(evx_batch *b, int *kernel_launches, float *device_ms);

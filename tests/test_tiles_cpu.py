@@ -7,7 +7,7 @@ import subprocess
 
 import pytest
 
-from everest_b200 import build
+from everest_b200 import autotune, build
 
 INT_MAX = 2**31 - 1
 MAX_EDGES = 2**30 - 2
@@ -51,3 +51,9 @@ def test_tile_numbers_fit(tiles, k, queries, roots, bps):
 
 def test_no_room(tiles):
     assert tiles.roots_of(4, 1000, 1, 1 << 30, 64) == 0
+
+
+def test_tuned_batch_tiles_differ(tiles):
+    # what the tuner times are different tilings of a range that fills the GPU
+    got = [tiles.roots_of(3, 1 << 30, 64, 5920, most) for most in autotune.BATCH_TILES]
+    assert got == list(autotune.BATCH_TILES)
