@@ -313,8 +313,6 @@ int evx_batch_launch(evx_batch *b) {
     b->groups.insert(b->groups.end(), {k, beg, pos - beg, tiles, bps * b->num_sms, ps ? 1 : 0, tile_roots, way});
     launches += tiles > 0 ? 1 : 0;
   }
-  if ((int)b->groups.size() / kGroupWords > kCursors)
-    return fail(EVX_ERR_INVALID, "too many motif sizes in one batch");
   EVX_CUDA(b->sides.ready(g_spare, b->device, b->stream, (int)b->groups.size() / kGroupWords, side_streams(b)));
   EVX_CUDA(cudaEventRecord(b->ev0, b->stream));
   if (b->use_graph) {

@@ -1401,12 +1401,17 @@ int occ_k(int *bps) {
 // The kernels of this size: count or enumerate; with or without the pair-run
 // walk (PS: compiled out where no level needs it); the constrained variant (CS:
 // node / edge predicates and temporal gaps, always with the walk); and, to count
-// three to five edges, one per way of counting the last edge.
-#define EVX_TAIL_CASE(FN, T, ...)                                                        \
-  case T: return x.ps ? FN<K, false, T, true, false>(__VA_ARGS__) : FN<K, false, T, false, false>(__VA_ARGS__); \
-  case T | kQStrict:                                                                     \
-    return x.ps ? FN<K, false, T | kQStrict, true, false>(__VA_ARGS__)                   \
-                : FN<K, false, T | kQStrict, false, false>(__VA_ARGS__);
+// three to five edges, one per way of counting the last edge.  Three edges walk
+// with two of the ways only: the walked edge joins the root's nodes, so the last
+// one does too or maps a new node.
+#define EVX_TAIL_CASE(FN, T, WALKS, ...)                                                 \
+  case T:                                                                                \
+    if constexpr (WALKS) if (x.ps) return FN<K, false, T, true, false>(__VA_ARGS__);     \
+    if (!x.ps) return FN<K, false, T, false, false>(__VA_ARGS__);                        \
+    break;
+#define EVX_TAIL_CASES(FN, T, WALKS, ...)                                                \
+  EVX_TAIL_CASE(FN, T, WALKS, __VA_ARGS__)                                               \
+  EVX_TAIL_CASE(FN, T | kQStrict, WALKS, __VA_ARGS__)
 #define EVX_PICK(FN, ...)                                                                \
   constexpr int K = EVX_K;                                                               \
   if (x.cs) return x.enumerate ? FN<K, true, kTailAny, true, true>(__VA_ARGS__)          \
@@ -1415,11 +1420,11 @@ int occ_k(int *bps) {
                                : FN<K, true, kTailAny, false, false>(__VA_ARGS__);       \
   if constexpr (K >= 3 && K <= 5) {                                                      \
     switch (x.tail) {                                                                    \
-      EVX_TAIL_CASE(FN, kQInlineLast, __VA_ARGS__)                                       \
-      EVX_TAIL_CASE(FN, kQSamePair, __VA_ARGS__)                                         \
-      EVX_TAIL_CASE(FN, kQRevPair, __VA_ARGS__)                                          \
-      EVX_TAIL_CASE(FN, kQPairHash, __VA_ARGS__)                                         \
-      EVX_TAIL_CASE(FN, kQNewArith, __VA_ARGS__)                                         \
+      EVX_TAIL_CASES(FN, kQInlineLast, true, __VA_ARGS__)                                \
+      EVX_TAIL_CASES(FN, kQNewArith, true, __VA_ARGS__)                                  \
+      EVX_TAIL_CASES(FN, kQSamePair, K > 3, __VA_ARGS__)                                 \
+      EVX_TAIL_CASES(FN, kQRevPair, K > 3, __VA_ARGS__)                                  \
+      EVX_TAIL_CASES(FN, kQPairHash, K > 3, __VA_ARGS__)                                 \
       default: break;                                                                    \
     }                                                                                    \
   }                                                                                      \
