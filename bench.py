@@ -117,23 +117,6 @@ def measured_peaks():
     return 6650.0, "fallback"
 
 
-def profile_traffic():
-    """DRAM bytes (read + write) of the search kernel over one timed step
-    (its 36 launches, the unit `roofline.achieved` is computed on) from the
-    committed ncu summary (a line 'traffic_bytes_per_step: N'), or None."""
-    p = os.path.join(ROOT, "profiles", "search_kernel_bursty-7.8m.md")
-    if not os.path.exists(p):
-        return None
-    with open(p) as f:
-        for line in f:
-            if line.strip().startswith("traffic_bytes_per_step:"):
-                try:
-                    return float(line.split(":", 1)[1].strip().split()[0])
-                except ValueError:
-                    return None
-    return None
-
-
 class ClockSampler:
     """nvidia-smi clocks and throttle reasons sampled during the timed region."""
     FIELDS = ("clocks.sm,clocks.max.sm,clocks_event_reasons.hw_slowdown,"
@@ -379,11 +362,7 @@ def run_gpu_arm(args):
     step_ms, kern_ms, launches = [], [], 0
     with ClockSampler(dev) as clk:
         for _ in range(args.steps):
-            # an NVTX range per timed step, so that ncu can capture exactly
-            # its launches (--nvtx --nvtx-include timed_step/)
-            torch.cuda.nvtx.range_push("timed_step")
             ms, counts, kms, nl = device_step()
-            torch.cuda.nvtx.range_pop()
             per_query_ms = {q["name"]: round(w.last_stats()["device_ms"], 3) for q, w in zip(qs, workers)}
             step_ms.append(ms)
             kern_ms.append(kms)
@@ -427,7 +406,6 @@ def run_gpu_arm(args):
     peak, peak_kind = measured_peaks()
     kern_avg_ms = sum(kern_ms) / len(kern_ms)
     achieved = bytes_alg / (kern_avg_ms / 1e3) / 1e9
-    traffic = profile_traffic()
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "higher_is_better": True,
@@ -446,9 +424,7 @@ def run_gpu_arm(args):
                              for k, c in tuned.items()},
         "edges_visited_per_s": world * cands / (ms_per_step / 1e3),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": traffic,
-                     "traffic_unit": "DRAM bytes read + written by the search kernel over one step "
-                                     "(36 launches), from one ncu capture of the timed step",
+                     "frac": achieved / peak, "traffic": None,  # DRAM bytes are not counted in a timed run
                      "peak_source": f"{peak_kind} hbm_gbs",
                      "model": "bytes_alg = 12 roots + 8 r_reads + 16 candidates of the serial "
                               "reference semantics, summed over the 36 queries"},
