@@ -760,9 +760,12 @@ int evx_worker_launch(evx_worker *w) {
   if ((int64_t)a.root_end + warps * (int64_t)a.roots_per_fetch >= (int64_t)INT_MAX)
     return fail(EVX_ERR_OVERFLOW, "root cursor would overflow int32");
   if (w->cons_active) return launch_constrained_job(w);
-  // (a search clears the state it leaves; other jobs and failed launches do not)
+  // (a search clears the state it leaves; other jobs, failed launches and a reset
+  // that is only captured, and may never run, do not)
   int launches = 0;
+  cudaStreamCaptureStatus captured = cudaStreamCaptureStatusNone;
   if (!w->state_clean) {
+    EVX_CUDA(cudaStreamIsCapturing(w->stream, &captured));
     reset_state_kernel<<<1, 1, 0, w->stream>>>(w->state_d, 0);
     EVX_CUDA(cudaGetLastError());
     launches++;
@@ -782,7 +785,7 @@ int evx_worker_launch(evx_worker *w) {
                              cudaMemcpyDeviceToHost, w->stream));
   }
   EVX_CUDA(cudaEventRecord(w->ev1, w->stream));
-  w->state_clean = true;
+  w->state_clean = captured == cudaStreamCaptureStatusNone;
   w->last_launches = launches;
   w->launched = true;
   return EVX_OK;
