@@ -273,7 +273,11 @@ int evx_batch_launch(evx_batch *b) {
   // so it has one per size: 64 requests over windows of 1000 roots, 4 blocks
   // per SM, 0.96 ms with one per way and 0.78 with one per size)
   const bool one = !side_streams(b);
-  const auto tail = [one](const QueryDesc &q) { return one ? kTailAny : tail_of(q.plan.k, q.flags); };
+  long long size_roots[EVX_MAX_MOTIF_EDGES + 1] = {};
+  for (const QueryDesc &q : b->queries) size_roots[q.plan.k] += q.root_end - q.root_beg;
+  const auto tail = [&](const QueryDesc &q) {
+    return one ? kTailAny : tail_of(q.plan.k, q.flags, size_roots[q.plan.k]);
+  };
   b->order.resize(nq);
   for (int i = 0; i < nq; i++) b->order[i] = i;
   std::stable_sort(b->order.begin(), b->order.end(), [&](int x, int y) {

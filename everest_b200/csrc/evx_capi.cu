@@ -750,8 +750,8 @@ int evx_worker_launch(evx_worker *w) {
   if (bps <= 0) {
     const int qf = (a.strict_ts ? kQStrict : 0) | a.tail_flags;
     const bool cs = cons_any(a.cons);
-    int rc = search_occupancy(w->plan.k, qf, a.enumerate != 0, cs || plan_pair_scan(w->plan, qf, a.enumerate != 0),
-                              cs, w->block, &bps);
+    int rc = search_occupancy(w->plan.k, qf, a.root_end - a.root_beg, a.enumerate != 0,
+                              cs || plan_pair_scan(w->plan, qf, a.enumerate != 0), cs, w->block, &bps);
     if (rc) return rc;
     if (bps <= 0) bps = 1;
   }

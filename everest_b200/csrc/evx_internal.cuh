@@ -297,19 +297,21 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
                   int grid, int block, cudaStream_t stream);
 // Launch a persistent search over a table of queries (count mode); q0 is
 // used when nq == 1.  Every query of the table has k edges and, unless tail is
-// tail_of(k, -1), counts its last edge in the way tail.
+// kTailAny, counts its last edge in the way tail.
 int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, int k, int tail, bool ps, int grid,
                  cudaStream_t stream);
 int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm);
-// The way of counting the last edge that a k-edge kernel with these flags is
-// compiled for (the same negative value for every kernel that holds all ways).
-int tail_of(int k, int qflags);
+// The way of counting the last edge of the kernel that a k-edge launch over so
+// many roots takes with these flags (kTailAny: the one that holds all ways).
+int tail_of(int k, int qflags, long long roots);
+constexpr int kFewRoots = 148 * 16;  // (every kernel holds 16 warps per SM or more)
 // Whether a query with these kQ flags walks a pair run at some level (the
 // kernels are compiled with and without that walk).
 bool plan_pair_scan(const MotifPlan &plan, int qflags, bool enumerate);
-// Max resident blocks per SM for a given motif size / kQ flags / mode /
+// Max resident blocks per SM for a given motif size / kQ flags / roots / mode /
 // pair-run variant / constrained variant (cs) / block.
-int search_occupancy(int k, int qflags, bool enumerate, bool ps, bool cs, int block, int *blocks_per_sm);
+int search_occupancy(int k, int qflags, long long roots, bool enumerate, bool ps, bool cs, int block,
+                     int *blocks_per_sm);
 // Whether search args carry constraints (the CS kernel variant runs them).
 inline bool cons_any(const ConsArgs &c) { return c.node_ok || c.edge_ok || c.has_gap; }
 

@@ -86,7 +86,8 @@ int launch_search(const GraphView &g, const MotifPlan &plan, const SearchArgs &a
   la.state = args.state;
   la.out = args.out;
   la.cons = args.cons;
-  const SearchKernel x{enumerate, plan_pair_scan(plan, q0.flags, enumerate), cons_any(args.cons), q0.flags & kTailFlags};
+  const SearchKernel x{enumerate, plan_pair_scan(plan, q0.flags, enumerate), cons_any(args.cons),
+                       tail_of(k, q0.flags, n)};
   return launch(k, x, g, q0, la, ea, grid, stream);
 }
 
@@ -97,20 +98,30 @@ int launch_table(const GraphView &g, const QueryDesc &q0, const LaunchArgs &la, 
   return launch(k, SearchKernel{false, ps, false, tail}, g, q0, la, ea, grid, stream);
 }
 
-int search_occupancy(int k, int qflags, bool enumerate, bool ps, bool cs, int block, int *blocks_per_sm) {
+int search_occupancy(int k, int qflags, long long roots, bool enumerate, bool ps, bool cs, int block,
+                     int *blocks_per_sm) {
   (void)block;
-  return occupancy(k, SearchKernel{enumerate, ps, cs, qflags & kTailFlags}, blocks_per_sm);
+  return occupancy(k, SearchKernel{enumerate, ps, cs, tail_of(k, qflags, roots)}, blocks_per_sm);
 }
 
 int table_occupancy(int k, int tail, bool ps, int *blocks_per_sm) {
   return occupancy(k, SearchKernel{false, ps, false, tail}, blocks_per_sm);
 }
 
-int tail_of(int k, int qflags) {
+// A launch of fewer roots than warps ends with its heaviest roots, each alone on
+// its warp, where the kernels with every way, at more registers and fewer blocks
+// per SM, go faster: requests over windows of 1000 roots of 63M edges, per way
+// and with every way, five edges with a pair-table last edge 8918 / 7987 ms (23
+// requests), a new node 6086 / 4964 (113), a fixed pair 1471 / 1361 (442); four
+// edges with a new node 282 / 244 (320), but a fixed pair 123 / 151 (42).  Over
+// 20k roots of 7.8M edges both are even, over all of 1.3M edges one way takes 10
+// to 25 % less.
+int tail_of(int k, int qflags, long long roots) {
   const int t = qflags & kTailFlags, way = t & ~kQStrict;
   const bool one =
       way == kQInlineLast || way == kQSamePair || way == kQRevPair || way == kQPairHash || way == kQNewArith;
-  return k >= 3 && k <= 5 && one ? t : kTailAny;
+  const bool few = roots < kFewRoots && (k == 5 || (k == 4 && way == kQNewArith));
+  return k >= 3 && k <= 5 && one && !few ? t : kTailAny;
 }
 
 }  // namespace evx
