@@ -132,23 +132,29 @@ int tail_mode(const MotifPlan &plan, unsigned flags, bool enumerate) {
 
 // The per-root window bound costs a gather and a gallop per root, and saves
 // scans.  Three edges whose last one is counted by range arithmetic have too
-// little left to save: on 7.8M edges, without and with it, 12 fixed-pair
-// queries 4.87 / 5.87 ms, 8 new-node 3.96 / 4.55, 4 same-pair 3.40 / 3.60, 4
-// reverse-pair 3.67 / 3.81; with a pair-table last edge 10.66 / 8.50, with four
-// edges 78 / 62 ms.  (Jobs with a work limit keep the bound: their meter counts
-// the records inside the windows it leaves.)
+// little left to save: on 7.8M bursty edges at a day, without and with it, 12
+// fixed-pair queries 4.95 / 5.86 ms, 8 new-node 3.95 / 4.43, 4 same-pair 3.32 /
+// 3.51, 4 reverse-pair 3.58 / 3.71 (at an hour 3.43 / 4.02, 2.87 / 3.13, 1.57 /
+// 1.62, 1.72 / 1.68); with a pair-table last edge 10.46 / 8.35, with four edges
+// 78 / 62 ms.  On 200k uniform edges it would save up to 8 % (new-node at an
+// hour .443 / .417).  (Jobs with a work limit keep the bound: their meter counts
+// the records inside the windows it leaves.  So do jobs that ask for it.)
 int bound_rule(const MotifPlan &plan, int qflags) {
   const int cheap = kQInlineLast | kQSamePair | kQRevPair | kQNewArith;
   return plan.k == 3 && (qflags & cheap) && !(qflags & kQKeepBound) ? qflags | kQNoBound : qflags;
 }
 
-// Rounds between rebalances where the caller does not say.  On 7.8M edges, every
-// 4 and every 16 rounds: three edges by range arithmetic 17.8 / 20.5 ms and by
-// the pair table 8.50 / 9.18, four edges 61.8 / 65.2, five no difference; but
-// four edges by the pair table 29.9 / 26.5 (the 4-cycle's windows are short).
+// Rounds between rebalances where the caller does not say.  Every 4 and every 16
+// rounds, on 7.8M bursty edges at a day: three edges with a fixed pair 4.95 /
+// 6.75 ms, same pair 3.32 / 4.59, reverse pair 3.58 / 4.86, pair table 8.35 /
+// 9.05, new node 3.95 / 3.85; four edges 61.8 / 65.2 (at an hour and on smaller
+// graphs within 5 %, but the fixed pair on 200k uniform edges .635 / .514); four
+// edges by the pair table 29.9 / 26.5 (the 4-cycle's windows are short).  Five
+// edges, on 1.3M edges: 64.1 / 62.0, requests of a few heavy roots up to 15 %
+// less at 16.
 int steal_rule(const MotifPlan &plan, int qflags) {
   const int arith = kQInlineLast | kQSamePair | kQRevPair | kQNewArith;
-  return plan.k >= 3 && plan.k <= 5 && (qflags & (plan.k == 4 ? arith : arith | kQPairHash)) ? 4 : 16;
+  return (plan.k == 3 && (qflags & (arith | kQPairHash))) || (plan.k == 4 && (qflags & arith)) ? 4 : 16;
 }
 
 }  // namespace evx
