@@ -281,19 +281,21 @@ static int alloc_graph(int device, int64_t E, int64_t V, evx_graph **out, cudaSt
 }
 
 // Checks and packs the host-format arrays on the device; *scratch (for
-// finish_graph) holds the time range, the list flags and the list nodes.
+// finish_graph) holds the time range, the flags and the lists' arrays.
 static ListScratch list_scratch(const DeviceGraph &g, int *scratch) {
-  return ListScratch{scratch + 32, scratch + 32 + g.num_edges, scratch + 2, scratch + 3};
+  int *lists = scratch + 32;
+  return ListScratch{lists, lists + g.num_edges, lists + 2 * g.num_edges, scratch + 2, scratch + 3, scratch + 4};
 }
 
 static int start_graph(evx_graph *h, const int *eg_d, const int *out_v_d, const int *in_v_d, const int *out_r_d,
                        const int *in_r_d, const int *euid_d, int **scratch, cudaStream_t s) {
   DeviceGraph &g = h->g;
-  int rc = validate_graph(g.device, g.num_edges, g.num_vertices, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, s);
-  if (rc) return rc;
-  EVX_CUDA(dev_alloc((void **)scratch, (32 + 2 * (size_t)g.num_edges) * sizeof(int), g.device, s));
+  EVX_CUDA(dev_alloc((void **)scratch, (32 + 3 * (size_t)g.num_edges) * sizeof(int), g.device, s));
   EVX_CUDA(cudaMemsetAsync(*scratch, 0, 32 * sizeof(int), s));
-  return pack_graph(g, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, euid_d, list_scratch(g, *scratch), s);
+  const ListScratch lists = list_scratch(g, *scratch);
+  int rc = validate_graph(g, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, lists, s);
+  if (rc) return rc;
+  return pack_graph(g, eg_d, out_v_d, in_v_d, out_r_d, in_r_d, euid_d, lists, s);
 }
 
 static int finish_graph(evx_graph *h, int *scratch, cudaStream_t s) {

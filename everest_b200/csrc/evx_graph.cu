@@ -82,14 +82,18 @@ __global__ void pack_nodes_kernel(const int *__restrict__ out_r, const int *__re
 }
 
 // Input checks: edge ids in [0, E), vertex ids in [0, V), timestamps sorted,
-// CSR offsets monotone from 0 to E.  Bits of *err name the failed check.
+// CSR offsets monotone from 0 to E.  Bits of *err name the failed check.  The
+// list positions start at -1 here too (two fills of their own took 5 us of a
+// small graph's load).
 __global__ void validate_kernel(const int *__restrict__ eg, const int *__restrict__ out_v,
                                 const int *__restrict__ in_v, const int *__restrict__ out_r,
-                                const int *__restrict__ in_r, int E, int V, int *err) {
+                                const int *__restrict__ in_r, int *__restrict__ outpos, int *__restrict__ inpos,
+                                int E, int V, int *err) {
   const int n = max(E, V + 1);
   int bad = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (i < E) {
+      outpos[i] = inpos[i] = -1;
       if ((unsigned)out_v[i] >= (unsigned)E || (unsigned)in_v[i] >= (unsigned)E) bad |= 1;
       if ((unsigned)eg[3 * i] >= (unsigned)V || (unsigned)eg[3 * i + 1] >= (unsigned)V) bad |= 2;
       if (i > 0 && eg[3 * i + 2] < eg[3 * i - 1]) bad |= 4;
@@ -135,33 +139,25 @@ int pack_graph(DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *i
   EVX_CUDA(cudaMemsetAsync(g.sig_in, 0, sizeof(unsigned long long) * (size_t)(V > 0 ? V : 1), s));
   if (V > 0) pack_nodes_kernel<<<grid, block, 0, s>>>(out_r_d, in_r_d, g.node_rng, (int)V);
   if (E > 0) {
-    int *outpos = nullptr;  // edges[].w, staged
-    EVX_CUDA(dev_alloc((void **)&outpos, sizeof(int) * (size_t)E, g.device, s));
-    EVX_CUDA(cudaMemsetAsync(outpos, 0xff, sizeof(int) * (size_t)E, s));
-    EVX_CUDA(cudaMemsetAsync(g.inpos, 0xff, sizeof(int) * (size_t)E, s));
-    scatter_pos_kernel<<<grid, block, 0, s>>>(out_v_d, in_v_d, outpos, g.inpos, (int)E);
-    pack_edges_kernel<<<grid, block, 0, s>>>(eg_d, euid_d, outpos, g.inpos, g.edges, g.euid, lists.lost, (int)E);
+    scatter_pos_kernel<<<grid, block, 0, s>>>(out_v_d, in_v_d, lists.outpos, g.inpos, (int)E);
+    pack_edges_kernel<<<grid, block, 0, s>>>(eg_d, euid_d, lists.outpos, g.inpos, g.edges, g.euid, lists.lost, (int)E);
     pack_rec_kernel<<<grid, block, 0, s>>>(out_v_d, in_v_d, g.edges, g.inpos, g.node_rng, g.out_rec,
                                            g.in_rec, g.sig_out, g.sig_in, lists, (int)E);
-    dev_free(outpos, s);
   }
   EVX_CUDA(cudaGetLastError());
   return EVX_OK;
 }
 
-int validate_graph(int device, int64_t E, int64_t V, const int *eg_d, const int *out_v_d, const int *in_v_d,
-                   const int *out_r_d, const int *in_r_d, cudaStream_t s) {
-  int *err = nullptr;
-  EVX_CUDA(dev_alloc((void **)&err, sizeof(int), device, s));
-  EVX_CUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+int validate_graph(const DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *in_v_d,
+                   const int *out_r_d, const int *in_r_d, const ListScratch &lists, cudaStream_t s) {
   int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  validate_kernel<<<sms * 8, 256, 0, s>>>(eg_d, out_v_d, in_v_d, out_r_d, in_r_d, (int)E, (int)V, err);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g.device);
+  validate_kernel<<<sms * 8, 256, 0, s>>>(eg_d, out_v_d, in_v_d, out_r_d, in_r_d, lists.outpos, g.inpos,
+                                          (int)g.num_edges, (int)g.num_vertices, lists.err);
   int h = 0;
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, lists.err, sizeof(int), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  dev_free(err, s);
   if (e != cudaSuccess) return cuda_fail(e, "graph validation");
   if (h & 1) return fail(EVX_ERR_INVALID, "edge id out of range in out/in lists");
   if (h & 2) return fail(EVX_ERR_INVALID, "vertex id out of range in Eg");

@@ -346,12 +346,13 @@ int cons_check_program(const evx_program &p, int num_vars, const char *what);
 int cons_build_masks(const evx_constraints &c, int n, const int *node_feat, int V, const int *edge_feat,
                      int E, unsigned short *node_ok, unsigned char *edge_ok, int num_sms, cudaStream_t s);
 
-// What packing leaves for the pair index build: the node of each position of
-// the out- and in-lists, whether an in-list entry is out of place, and whether
-// a list lacks an edge.
+// Scratch of a graph's build: what checking leaves for packing (each edge's
+// position in the out-lists, the failed checks) and packing for the pair index
+// (the node of each position of the out- and in-lists, whether an in-list entry
+// is out of place, and whether a list lacks an edge).
 struct ListScratch {
-  int *out_node, *in_node;  // [E]
-  int *stray, *lost;
+  int *out_node, *in_node, *outpos;  // [E]
+  int *stray, *lost, *err;           // zero before
 };
 
 // Build the pair index (defined in evx_pairs.cu); needs the packed graph.
@@ -360,11 +361,11 @@ int build_pair_index(DeviceGraph &g, const ListScratch &lists, bool in_grouped, 
 
 // Check the host-format arrays on the device before anything indexes with
 // them (evx_graph.cu); returns EVX_ERR_INVALID with a message on bad input.
-int validate_graph(int device, int64_t E, int64_t V, const int *eg_d, const int *out_v_d, const int *in_v_d,
-                   const int *out_r_d, const int *in_r_d, cudaStream_t s);
+int validate_graph(const DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *in_v_d,
+                   const int *out_r_d, const int *in_r_d, const ListScratch &lists, cudaStream_t s);
 
 // Build the packed device layout from the uploaded host-format arrays
-// (defined in evx_graph.cu) and fill lists (*lists.stray, *lists.lost: zero before).
+// (defined in evx_graph.cu) and fill lists.
 int pack_graph(DeviceGraph &g, const int *eg_d, const int *out_v_d, const int *in_v_d,
                const int *out_r_d, const int *in_r_d, const int *euid_d, const ListScratch &lists, cudaStream_t s);
 
