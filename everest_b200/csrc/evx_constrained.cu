@@ -124,7 +124,7 @@ int cons_check_program(const evx_program &p, int num_vars, const char *what) {
 __global__ void __launch_bounds__(256) cons_node_mask_kernel(const int *__restrict__ feat, int V, int n,
                                                              const __grid_constant__ evx_constraints c,
                                                              unsigned short *__restrict__ out) {
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < V; x += gridDim.x * blockDim.x) {
+  for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < (unsigned)V; x += gridDim.x * blockDim.x) {
     const long long f = __ldg(feat + x);
     auto var = [&](int) { return f; };
     unsigned m = 0;

@@ -33,7 +33,8 @@ __global__ void pack_edges_kernel(const int *__restrict__ eg, const int *__restr
   bool bad = false;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int at = outpos[i];
-    edges[i] = make_int4(eg[3 * i], eg[3 * i + 1], eg[3 * i + 2], at);
+    const int *e = eg + 3ll * i;
+    edges[i] = make_int4(e[0], e[1], e[2], at);
     euid[i] = euid_in ? euid_in[i] : i;
     bad |= at < 0 || inpos[i] < 0;
   }
@@ -76,7 +77,7 @@ __global__ void pack_rec_kernel(const int *__restrict__ out_v, const int *__rest
 
 __global__ void pack_nodes_kernel(const int *__restrict__ out_r, const int *__restrict__ in_r,
                                   int4 *__restrict__ node_rng, int nv) {
-  for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < nv; x += gridDim.x * blockDim.x) {
+  for (unsigned x = blockIdx.x * blockDim.x + threadIdx.x; x < (unsigned)nv; x += gridDim.x * blockDim.x) {
     node_rng[x] = make_int4(out_r[x], out_r[x + 1], in_r[x], in_r[x + 1]);
   }
 }
@@ -91,14 +92,15 @@ __global__ void validate_kernel(const int *__restrict__ eg, const int *__restric
                                 int E, int V, int *err) {
   const int n = max(E, V + 1);
   int bad = 0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (i < E) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < (unsigned)n; i += gridDim.x * blockDim.x) {
+    if (i < (unsigned)E) {
+      const int *e = eg + 3ll * i;
       outpos[i] = inpos[i] = -1;
       if ((unsigned)out_v[i] >= (unsigned)E || (unsigned)in_v[i] >= (unsigned)E) bad |= 1;
-      if ((unsigned)eg[3 * i] >= (unsigned)V || (unsigned)eg[3 * i + 1] >= (unsigned)V) bad |= 2;
-      if (i > 0 && eg[3 * i + 2] < eg[3 * i - 1]) bad |= 4;
+      if ((unsigned)e[0] >= (unsigned)V || (unsigned)e[1] >= (unsigned)V) bad |= 2;
+      if (i > 0 && e[2] < e[-1]) bad |= 4;
     }
-    if (i < V && (out_r[i + 1] < out_r[i] || in_r[i + 1] < in_r[i])) bad |= 8;
+    if (i < (unsigned)V && (out_r[i + 1] < out_r[i] || in_r[i + 1] < in_r[i])) bad |= 8;
     if (i == 0 && (out_r[0] != 0 || in_r[0] != 0 || out_r[V] != E || in_r[V] != E)) bad |= 16;
   }
   if (bad) atomicOr(err, bad);

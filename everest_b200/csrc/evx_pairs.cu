@@ -110,8 +110,8 @@ __global__ void pair_dir_kernel(const unsigned long long *__restrict__ ukeys,
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, dt = gridDim.x * blockDim.x;
   for (int r = t0; r <= P; r += dt)
     dir[r] = r == P ? make_int2(0x7fffffff, n_edges) : make_int2((int)(unsigned)(ukeys[r] & 0xffffffffull), starts[r]);
-  for (int x = t0; x <= nv; x += dt) {
-    const unsigned long long k = pair_key(x, 0);
+  for (unsigned x = t0; x <= (unsigned)nv; x += dt) {
+    const unsigned long long k = pair_key((int)x, 0);
     int lo = 0, hi = P;
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
