@@ -83,7 +83,7 @@ def parse():
     ap.add_argument("--flags", type=int, default=0, help="with --motif / --constrained-query: EVX_FLAG_* bits")
     ap.add_argument("--mode", default="single", choices=["single", "batch", "serve", "enumerate", "constrained"],
                     help="single: the 36-query per-query-kernel step (default); batch: 64 mixed queries "
-                         "in one persistent launch per motif size vs the same queries one at a time; serve: "
+                         "in a few persistent launches vs the same queries one at a time; serve: "
                          "the serving loop (saturated and Poisson arrivals) vs one at a time; enumerate: "
                          "the 36M-edge 4-cycle at cap 1e6 with a host check of the rows; constrained: the "
                          "reference's node / temporal / anti-edge / filter query shapes on the 7.8M graph")

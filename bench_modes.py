@@ -72,8 +72,8 @@ def _pct(x, p):
 def batch_leg(window: int = 0, n: int = 64, limit: int = 0, warmup: int = 1, steps: int = 1,
               tune: bool = False, tile: int = 64) -> dict:
     """C3: n random connected 3/4-edge patterns on 2-4 nodes, delta cycling
-    3600 / 86400 / 604800, on the 2.6M-node / 36M-edge graph, in one
-    persistent launch per motif size replayed from a CUDA graph, against the
+    3600 / 86400 / 604800, on the 2.6M-node / 36M-edge graph, in
+    persistent launches side by side replayed from a CUDA graph, against the
     same queries one at a time through the per-query kernel
     (evx_worker_take + evx_worker_run each).  window = 0: every root of the
     graph (C3 as specified); else a random window of that many roots per
