@@ -129,7 +129,7 @@ constexpr int kQKeepBound = 1024;  // host only: that bound whatever bound_rule 
 // How a kernel counts the last edge: its kQ* bit, with kQStrict or not, where
 // that is compiled in (count mode, no constraints), kTailAny where the query's
 // flags say (everything else).  A kernel that holds every way spills
-// (196 bytes of stores for 3 edges, 0 to 88 with one way), and its dead paths
+// (196 bytes of stores for 3 edges, 0 to 120 with one way), and its dead paths
 // cost issue slots: the 36 three-edge queries on 7.8M edges 37.2 -> 30.2 ms.
 constexpr int kTailFlags = kQStrict | kQInlineLast | kQSamePair | kQRevPair | kQPairHash | kQPairDir | kQNewArith;
 constexpr int kTailAny = -1;
