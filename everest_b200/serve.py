@@ -124,7 +124,7 @@ class Server:
                 w.set_limit(self.limit)
         # an enumeration's kernel holds its blocks until it ends: while count
         # work is queued or running, run it on a fraction of the SMs
-        # (blocks_per_sm of the usual 4-8) so that count batches still find
+        # (blocks_per_sm of the usual 4-10) so that count batches still find
         # room; with no count work about, on the whole GPU
         self.enum_blocks_per_sm = int(enum_blocks_per_sm)
         self.enum_reqs: List[Optional[Request]] = [None] * enum_slots
@@ -315,9 +315,7 @@ class Server:
     def _admit(self) -> bool:
         progressed = False
         # count queries: fill free batch slots.  A batch holds one graph and
-        # one motif size: the persistent kernel is instantiated for the
-        # largest motif of its batch, and a smaller motif run in a larger
-        # instantiation pays for its registers and shared memory.
+        # one motif size, whose kernels' resident blocks its share is of.
         for i, b in enumerate(self.batches):
             if self.batch_reqs[i] is not None:
                 continue
